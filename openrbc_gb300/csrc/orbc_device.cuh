@@ -97,9 +97,11 @@ template<class R> struct BondP {
 template<class R> struct FFDev {
     PairP<R> pair[NT * NT];        // by (ti * NT + tj)
     R mass[NT], inv_mass[NT], gamma[NT], sigma[NT];
+    R reach2[NT];                  // the largest interaction range^2 of the type with any other
     BondP<R> bond[MAX_BT];
     float rlist2[16 * 16];          // neighbour-list cutoff^2 (cut + skin)^2, 0 = never
-    float rin2[16 * 16];            // interaction range^2: list entries inside it go to the inner rows
+    float rin2[16 * 16];            // interaction range^2 of the anisotropic pairs with a lipid partner: list entries
+                                    // inside it go to the inner rows (0 for the other pairs: always shell rows)
 };
 
 struct SysDev {
@@ -154,8 +156,8 @@ struct SysState {
     double pad;
 };
 
-struct Scalars {
-    int cur, lp, rebuild, error;
+struct __align__(16) Scalars {
+    int cur, lp, rebuild, error;  // read together (halted)
     int max_nnb, out_of_grid, cond_hint;
     int nh_half;          // 1 between a Nose-Hoover first half and its second half
     unsigned int blk_counter, mesh_counter;
@@ -173,6 +175,11 @@ struct Scalars {
  * kernel reads the same value. */
 __device__ __forceinline__ bool halted(const Scalars *S) {
     return (__ldcg(&S->error) & (ERRB_NBR_OVERFLOW | ERRB_GRID)) != 0;
+}
+
+/* the same from the first four words of Scalars (cur, lp, rebuild, error) in one load */
+__device__ __forceinline__ bool halted(const int4 &head) {
+    return (head.w & (ERRB_NBR_OVERFLOW | ERRB_GRID)) != 0;
 }
 
 template<class R> struct KArgs {
@@ -211,13 +218,11 @@ template<class R> struct KArgs {
     R skin_half2;
     uint64_t seed;
     int rebuild_every;
-    int variant;             // force-kernel form (see launch_step_langevin)
+    int kahan;               // compensated sums of each particle's force and torque
     int carry_forces;        // forces / torques persist between kernels (Nose-Hoover)
     int zero_bulk;           // remove the mean lipid velocity before integrating
     int nlist_lane;          // list-build form: 0 per cell of a warp, 1 per-lane 27-cell sweep, 2 two-phase
     const FFDev<R> *ff;      // force-field tables (global)
-    PairP<R> ll;             // the lipid-lipid pair, in kernel-parameter space: read as constant operands,
-                             // so the bulk pair path keeps no registers for its parameters
 };
 
 // host-side launchers (explicitly instantiated for float and double)

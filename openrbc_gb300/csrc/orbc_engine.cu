@@ -1750,6 +1750,7 @@ template<class R> class Engine : public EngineBase {
             hff.gamma[t] = R(gam);
             hff.sigma[t] = R(sig);
         }
+        for (int k = 0; k < NT * NT; ++k) hff.reach2[k / NT] = std::max(hff.reach2[k / NT], hff.pair[k].anysq);
         for (int b = 0; b < MAX_BT; ++b) {
             hff.bond[b].K = R(P.bond_K[b]);
             hff.bond[b].Rm = R(P.bond_R[b]);
@@ -1762,7 +1763,8 @@ template<class R> class Engine : public EngineBase {
                 if (ti < NT && tj < NT && F.range[ti * NT + tj] > 0) {
                     const double rl = F.range[ti * NT + tj] + P.skin;
                     v = float(rl * rl);
-                    vin = float(F.range[ti * NT + tj] * F.range[ti * NT + tj]);
+                    if (tj == 0 && F.kind[ti * NT + tj] == PAIR_ANISO)
+                        vin = float(F.range[ti * NT + tj] * F.range[ti * NT + tj]);
                 }
                 hff.rlist2[ti * 16 + tj] = v;
                 hff.rin2[ti * 16 + tj] = vin;
@@ -1817,12 +1819,11 @@ template<class R> class Engine : public EngineBase {
         a.skin_half2 = R(0.25 * P.skin * P.skin);
         a.seed = P.seed;
         a.rebuild_every = P.rebuild_every;
-        a.variant = P.kernel_variant & (7 | 32 | 64);
+        a.kahan = (P.kernel_variant & 64) ? 1 : 0;
         a.nlist_lane = (P.kernel_variant >> 3) & 3;
         a.carry_forces = P.integrator == ORBC_INT_NOSE_HOOVER ? 1 : 0;
         a.zero_bulk = P.zero_bulk ? 1 : 0;
         a.ff = ffd.p;
-        a.ll = hff.pair[0];
     }
 
     int build_lists(bool first) {

@@ -21,6 +21,8 @@
 // k_advance flips the buffers.
 #include "orbc_device.cuh"
 
+#include <type_traits>
+
 namespace orbc {
 
 namespace {
@@ -148,7 +150,7 @@ __device__ __forceinline__ void repf(const PairP<R> &P, R dx, R dy, R dz, R r2, 
 
 /* Dispatch of src/compute_pairwise_fused.h:91-236 for a non lipid-lipid pair. */
 template<class R, bool E>
-__device__ __forceinline__ void pair_general_body(const PairP<R> &P, R dx, R dy, R dz, R r2, R nix, R niy, R niz,
+__device__ __forceinline__ void pair_general(const PairP<R> &P, R dx, R dy, R dz, R r2, R nix, R niy, R niz,
                                                   R njx, R njy, R njz, R3<R> &f, R3<R> &t, R &e) {
     if (!(r2 > R(1e-5))) return;
     if (r2 < P.cutsq) {
@@ -160,21 +162,6 @@ __device__ __forceinline__ void pair_general_body(const PairP<R> &P, R dx, R dy,
         ljf<R, E>(P, dx, dy, dz, r2, f, e);
     }
 }
-template<class R, bool E>
-__device__ __noinline__ void pair_general_call(const PairP<R> &P, R dx, R dy, R dz, R r2, R nix, R niy, R niz,
-                                               R njx, R njy, R njz, R3<R> &f, R3<R> &t, R &e) {
-    pair_general_body<R, E>(P, dx, dy, dz, r2, nix, niy, niz, njx, njy, njz, f, t, e);
-}
-/* INL: inline the rare non-lipid path (more registers, no call) or call it. */
-template<class R, bool E, bool INL>
-__device__ __forceinline__ void pair_general(const PairP<R> &P, R dx, R dy, R dz, R r2, R nix, R niy, R niz, R njx,
-                                             R njy, R njz, R3<R> &f, R3<R> &t, R &e) {
-    if (INL)
-        pair_general_body<R, E>(P, dx, dy, dz, r2, nix, niy, niz, njx, njy, njz, f, t, e);
-    else
-        pair_general_call<R, E>(P, dx, dy, dz, r2, nix, niy, niz, njx, njy, njz, f, t, e);
-}
-
 __device__ __forceinline__ int wrap_delta(int d, int n) {
     if (2 * d >= n) return d - n;
     if (2 * d < -n) return d + n;
@@ -231,6 +218,127 @@ __device__ __forceinline__ R bond_kappa(const BondP<R> &B, R r0, R r, R &e, int 
     }
 }
 
+/* s += d with Kahan compensation c (one component). */
+template<class R> __device__ __forceinline__ void kahan_add(R &s, R &c, R d) {
+    const R y = d - c;
+    const R t = s + y;
+    c = (t - s) - y;
+    s = t;
+}
+
+/* The 27 cell shifts of the list entries, already multiplied by the cell
+ * size: x_i - x_j = (o_i - o_j) + shift(code) (a shift of -1, 0 or +1 cells
+ * times Lc is exact, so this rounds as the unscaled product would).  One table
+ * per warp (which never straddles two systems), one array per axis: three
+ * 4-byte lookups by 32 lanes are three conflict-free wavefronts of the L1 data
+ * pipe that the gathers need too, one 16-byte lookup takes more than five. */
+template<class R> struct ShiftTab {
+    R v[3][32];
+};
+template<class R> __device__ __forceinline__ void init_shift(const SysDev &sd, ShiftTab<R> &sh) {
+    const int lane = threadIdx.x & 31;
+    if (lane < 27) {
+        sh.v[0][lane] = R(-(lane % 3 - 1)) * lc_of<R>(sd, 0);
+        sh.v[1][lane] = R(-((lane / 3) % 3 - 1)) * lc_of<R>(sd, 1);
+        sh.v[2][lane] = R(-(lane / 9 - 1)) * lc_of<R>(sd, 2);
+    }
+    __syncwarp();
+}
+
+/* ------------------------------------------------------------------------- */
+/* Pair sums of a slot                                                       */
+/* ------------------------------------------------------------------------- */
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+
+/* 1/sqrt(r2) for 1e-5 <= r2: the hardware estimate in FP32; in FP64 one
+ * third-order step from it, y (1 + e/2 + 3 e^2 / 8) with e = 1 - r2 y^2: the
+ * error e of the estimate (3e-7) leaves 5 e^3 / 16 < 1e-20, below FP64
+ * rounding, in five FP64 operations. */
+__device__ __forceinline__ float rsqrt_pair(float r2) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r2));
+    return y;
+}
+__device__ __forceinline__ double rsqrt_pair(double r2) {
+    const double y = double(rsqrt_pair(float(r2)));
+    const double e = fma_rn(-mul_rn(r2, y), y, 1.0);
+    return fma_rn(mul_rn(fma_rn(e, 0.375, 0.5), e), y, y);
+}
+
+/* The anisotropic pair with a lipid j, by the owner's own parameters, in the
+ * form that keeps the neighbour's vectors outermost:
+ *   f = sum (cu d + kj n_j) + n_i sum kd,   t = sum (kd d - au n_j)
+ * with d = x_i - x_j, niu = n_i.d / r, nju = n_j.d / r and the coefficients of
+ * src/pairwise_kernel.h:30-68.  Pairs outside the range enter with r_c - r
+ * clamped to 0, so that every coefficient vanishes and no branch is needed.
+ * Each operation is rounded as written, so the sums do not depend on how the
+ * loops around them are compiled. */
+template<class R> struct OwnP {
+    R cut, rep8, a0, a1, aatt, hrep;  // a0 = 4 att (1 - alpha), a1 = 4 att alpha, hrep = rep / 2
+};
+constexpr int SHELL_U = 2;  // shell rows tested together
+template<class R> __device__ __forceinline__ OwnP<R> own_params(const PairP<R> &q) {
+    OwnP<R> P;
+    P.cut = q.cut;
+    P.rep8 = q.rep8;
+    P.a1 = q.att4 * q.alpha;
+    P.a0 = q.att4 - P.a1;
+    P.aatt = q.aatt;
+    P.hrep = R(0.5) * q.rep;
+    return P;
+}
+constexpr int NACC = 7;  // force (3), torque (3), coefficient of n_i
+template<class R, bool K> struct PairAcc {
+    R s[NACC], c[K ? NACC : 1], e;  // sums, Kahan compensations, energy
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int k = 0; k < NACC; ++k) s[k] = R(0);
+#pragma unroll
+        for (int k = 0; k < (K ? NACC : 1); ++k) c[k] = R(0);
+        e = R(0);
+    }
+};
+template<class R, bool E, bool K>
+__device__ __forceinline__ void pair_term(PairAcc<R, K> &A, const OwnP<R> &P, const R d[3], const R n[3], R nix, R niy,
+                                          R niz) {
+    const R r2 = fma_rn(d[2], d[2], fma_rn(d[1], d[1], mul_rn(d[0], d[0])));
+    const R r2c = r2 > R(1e-5) ? r2 : R(1e30);  // coinciding particles: no force, as outside the range
+    const R ri = rsqrt_pair(r2c);
+    const R rc = max(fma_rn(-r2c, ri, P.cut), R(0));
+    const R nn = fma_rn(niz, n[2], fma_rn(niy, n[1], mul_rn(nix, n[0])));
+    const R niu = mul_rn(fma_rn(niz, d[2], fma_rn(niy, d[1], mul_rn(nix, d[0]))), ri);
+    const R nju = mul_rn(fma_rn(n[2], d[2], fma_rn(n[1], d[1], mul_rn(n[0], d[0]))), ri);
+    const R A4 = fma_rn(mul_rn(niu, nju), -P.a1, fma_rn(nn, P.a1, P.a0));  // 4 att A
+    const R rc2 = mul_rn(rc, rc), rc4 = mul_rn(rc2, rc2);
+    const R fra = mul_rn(mul_rn(rc2, rc), fma_rn(P.rep8, rc4, A4));
+    const R au = mul_rn(P.aatt, rc4);
+    const R auar = mul_rn(au, ri);
+    const R kd = mul_rn(auar, nju), kj = mul_rn(auar, niu);
+    const R cu = mul_rn(fma_rn(kd, mul_rn(niu, R(-2)), fra), ri);
+    if (K) {
+#pragma unroll
+        for (int k = 0; k < NACC; ++k) {
+            const R t = k < 3   ? fma_rn(cu, d[k % 3], mul_rn(kj, n[k % 3]))
+                        : k < 6 ? fma_rn(kd, d[k % 3], -mul_rn(au, n[k % 3]))
+                                : kd;
+            kahan_add(A.s[k], A.c[k], t);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            A.s[k] = fma_rn(cu, d[k], fma_rn(kj, n[k], A.s[k]));
+            A.s[3 + k] = fma_rn(kd, d[k], fma_rn(-au, n[k], A.s[3 + k]));
+        }
+        A.s[6] = add_rn(A.s[6], kd);
+    }
+    if (E) A.e = fma_rn(rc4, fma_rn(P.hrep, rc4, mul_rn(A4, R(0.125))), A.e);  // half of rep rc^8 + A att rc^4
+}
+
 /* Bring the used rows of this warp's block of neighbour entries (read once
  * per step) into L1 ahead of the pair loops, so the loops' entry loads do not
  * wait on DRAM.  packed = inner count | shell count << 16.  All 32 lanes must
@@ -245,282 +353,268 @@ __device__ __forceinline__ void prefetch_warp_list(const uint32_t *nbr, int i, i
     }
 }
 
-/* The 27 cell shifts of the list entries, already multiplied by the block's
- * cell size: x_i - x_j = (o_i - o_j) + sh[code] (a shift of -1, 0 or +1 cells
- * times Lc is exact, so this rounds as the unscaled product would).  A block
- * never straddles two systems. */
-template<class R> __device__ __forceinline__ void init_shift(const KArgs<R> &a, typename Vec<R>::T4 *sh) {
-    if (threadIdx.x < 27) {
-        const SysDev &sd = a.sys[a.blk_sys[(blockIdx.x * blockDim.x) / SYS_PAD]];
-        const int c = threadIdx.x;
-        typename Vec<R>::T4 v;
-        v.x = R(-(c % 3 - 1)) * lc_of<R>(sd, 0);
-        v.y = R(-((c / 3) % 3 - 1)) * lc_of<R>(sd, 1);
-        v.z = R(-(c / 9 - 1)) * lc_of<R>(sd, 2);
-        v.w = R(0);
-        sh[c] = v;
-    }
-    __syncthreads();
+/* Resident blocks of LITE_BS threads asked of the force kernels: FP32, 16 at
+ * 64 registers for batches of two rows (14 with energy or compensated sums,
+ * which need more: EK), 10 for batches of four; the FP64 forms are bound by the FP64 pipe and
+ * keep all the registers they need. */
+template<class R, bool EK, int U> constexpr int force_blocks() {
+    return sizeof(R) == 8 ? 1 : U == 2 ? (EK ? 14 : 16) : 10;
 }
 
-/* Resident blocks of LITE_BS threads asked of the force kernels: the FP32
- * count, halved for FP64, whose doubles need twice the registers (the FP64
- * forms are bound by the FP64 pipe, so fewer resident warps cost nothing,
- * while spills would). */
-template<class R> constexpr int fp_blocks(int n) { return sizeof(R) == 4 ? n : n / 2; }
-
-/* Form bits of the force loop (orbc_params.kernel_variant; the autotuner
- * picks one per workload):
- *   1  software-pipelined list pass (the next entry's gathers in flight while
- *      the current pair is evaluated) instead of a 2-way unrolled loop;
- *   2  the rare non-lipid pair path inlined instead of called;
- *   4  occupancy form of the lite Langevin kernel (more resident blocks);
- *   32 merged shell pass: the skin-shell rows are only distance-tested, each
- *      lane records its hits in a bit mask, and the hits are evaluated in the
- *      same loop as the inner rows, so a shell row that one lane of a warp
- *      hits no longer costs the whole warp a pair evaluation; and where a
- *      lane's pair involves a protein, all lanes of the warp evaluate their
- *      lipid-lipid and lipid-protein pairs in one anisotropic code path with
- *      per-pair parameters instead of two paths one after the other.  The
- *      pairs are added in the same order as without it: the results are
- *      bit-identical;
- *   64 compensated accumulation: each particle's force and torque are summed
- *      with Kahan compensation (the rounding error of each running sum is
- *      carried into the next addition), for the FP32 form. */
-constexpr int FORM_PIPE = 1, FORM_INLINE = 2, FORM_OCC = 4, FORM_MERGED = 32, FORM_KAHAN = 64;
-
-/* s += d with Kahan compensation c (one component). */
-template<class R> __device__ __forceinline__ void kahan_add(R &s, R &c, R d) {
-    const R y = d - c;
-    const R t = s + y;
-    c = (t - s) - y;
-    s = t;
-}
-
-/* All forces and torques on particle slot i: pair terms over its neighbour
- * list (form V, above), bonds, mesh constraint. */
-template<class R, bool E, int V>
-__device__ __forceinline__ void particle_forces(const KArgs<R> &a, const FFDev<R> &F, int i, int cur, int lp, int w,
-                                                const typename Vec<R>::T4 &pi, const typename Vec<R>::T4 &ni,
-                                                const SysDev &sd, const SysState &ss,
-                                                const typename Vec<R>::T4 *sh, R3<R> &f, R3<R> &t, R &e,
-                                                int &flags) {
+/* Pair sums of slot i over its list.  Shell rows are tested first, 32 at a
+ * time; a hit is a bit of a mask.  Then the inner rows and the lipids among
+ * the hits go through one loop, U of them at a time: their entries and
+ * gathers are issued together and their terms added in row order, so the sums
+ * are the same for every U.  The hits that need the general pair table (a
+ * protein partner, or an owner whose pairs with lipids are not anisotropic:
+ * the list build puts all of these in the shell rows) follow.  All 32 lanes
+ * of the warp must call it. */
+template<class R, bool E, bool K, int U>
+__device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, const OwnP<R> &P, R lim, int own_gen,
+                                          int i, const typename Vec<R>::T4 *__restrict__ pos,
+                                          const typename Vec<R>::T4 *__restrict__ nrm, int ty, int packed,
+                                          const typename Vec<R>::T4 &pi, const typename Vec<R>::T4 &ni,
+                                          const ShiftTab<R> &sh, PairAcc<R, K> &A) {
     using T4 = typename Vec<R>::T4;
-    constexpr bool KAHAN = (V & FORM_KAHAN) != 0;
-    const int ty = w_type(w);
-    const T4 *__restrict__ pos = a.pos[cur];
-    const T4 *__restrict__ nrm = a.nrm[cur];
+    int nin = packed & 0xffff;
+    const int nout = packed >> 16;
     const uint32_t *__restrict__ nb = a.nbr + nbr_index(i, 0, a.cap);
-    const int packed = a.nnb[i];
-    const int nin = packed & 0xffff, nout = packed >> 16;
     const uint32_t *__restrict__ shell = nb + int64_t(a.cap - 1) * 32;  // shell rows run downwards
-    const int64_t stride = 32;
-    const R ll_cutsq = a.ll.cutsq;
-    R3<R> cf = {0, 0, 0}, ct = {0, 0, 0};  // Kahan compensations (KAHAN only)
-    auto accumulate = [&](const R3<R> &df, const R3<R> &dt) {
-        kahan_add(f.x, cf.x, df.x);
-        kahan_add(f.y, cf.y, df.y);
-        kahan_add(f.z, cf.z, df.z);
-        kahan_add(t.x, ct.x, dt.x);
-        kahan_add(t.y, ct.y, dt.y);
-        kahan_add(t.z, ct.z, dt.z);
+    const uint32_t self = uint32_t(i) | (13u << NB_SHIFT);              // distance 0: contributes nothing
+    auto offset = [&](uint32_t ent, const T4 &pj, R d[3]) {
+        const int c = int(ent >> NB_SHIFT);
+        d[0] = add_rn(add_rn(pi.x, -pj.x), sh.v[0][c]);
+        d[1] = add_rn(add_rn(pi.y, -pj.y), sh.v[1][c]);
+        d[2] = add_rn(add_rn(pi.z, -pj.z), sh.v[2][c]);
     };
-    auto pair = [&](uint32_t ent, const T4 &pj, const T4 &nj) {
-        const T4 s = sh[ent >> NB_SHIFT];
-        const R dx = (pi.x - pj.x) + s.x;
-        const R dy = (pi.y - pj.y) + s.y;
-        const R dz = (pi.z - pj.z) + s.z;
-        const R r2 = dx * dx + dy * dy + dz * dz;
-        const int tj = w_type(wbits(pj.w));
-        if (KAHAN) {
+    auto dist2 = [&](const R d[3]) { return fma_rn(d[2], d[2], fma_rn(d[1], d[1], mul_rn(d[0], d[0]))); };
+    auto term = [&](uint32_t ent, const T4 &pj, const T4 &nj) {
+        R d[3];
+        const R n[3] = {nj.x, nj.y, nj.z};
+        offset(ent, pj, d);
+        pair_term<R, E, K>(A, P, d, n, ni.x, ni.y, ni.z);
+    };
+    // rows that every lane still has inside (rounded down to whole batches): no selection
+    int kmin = int(__reduce_min_sync(0xffffffffu, unsigned(nin))) / U * U;
+    for (int k0 = 0;; k0 += 32) {
+        uint32_t hm = 0u, hb = 0u;
+        const int nq = min(32, nout - k0);
+        const int nqmax = int(__reduce_max_sync(0xffffffffu, unsigned(max(nq, 0))));
+        for (int k = 0; k < nqmax; k += SHELL_U) {
+            uint32_t ent[SHELL_U];
+            T4 pj[SHELL_U];
+#pragma unroll
+            for (int u = 0; u < SHELL_U; ++u) ent[u] = k + u < nq ? __ldg(shell - (k + u + k0) * 32) : self;
+#pragma unroll
+            for (int u = 0; u < SHELL_U; ++u) pj[u] = ldg4<R>(pos + (ent[u] & NB_MASK));
+#pragma unroll
+            for (int u = 0; u < SHELL_U; ++u) {
+                R d[3];
+                offset(ent[u], pj[u], d);
+                if (k + u < nq && dist2(d) < lim) hm |= 1u << (k + u);
+            }
+        }
+        const int total = int(__reduce_max_sync(0xffffffffu, unsigned(nin + __popc(hm))));
+        for (int k = 0; k < kmin; k += U) {
+            uint32_t ent[U];
+            T4 pj[U], nj[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) ent[u] = __ldg(nb + (k + u) * 32);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                pj[u] = ldg4<R>(pos + (ent[u] & NB_MASK));
+                nj[u] = ldg4<R>(nrm + (ent[u] & NB_MASK));
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) term(ent[u], pj[u], nj[u]);
+        }
+        for (int k = kmin; k < total; k += U) {
+            uint32_t ent[U], bit[U];
+            T4 pj[U], nj[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bool in = k + u < nin;
+                bit[u] = in ? 0u : hm & (0u - hm);
+                hm ^= bit[u];
+                const int row = in ? k + u : a.cap - 1 - k0 - (31 - __clz(int(bit[u])));
+                ent[u] = (in || bit[u]) ? __ldg(nb + row * 32) : self;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                pj[u] = ldg4<R>(pos + (ent[u] & NB_MASK));
+                nj[u] = ldg4<R>(nrm + (ent[u] & NB_MASK));
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int tj = w_type(wbits(pj[u].w));
+                if (bit[u] && (tj | own_gen) != 0) {
+                    // a lipid's pair with a protein has parameters of its own; the rest waits
+                    const PairP<R> &q = F.pair[ty * NT + tj];
+                    if (ty == 0 && q.kind == PAIR_ANISO) {
+                        R d[3];
+                        const R n[3] = {nj[u].x, nj[u].y, nj[u].z};
+                        offset(ent[u], pj[u], d);
+                        pair_term<R, E, K>(A, own_params(q), d, n, ni.x, ni.y, ni.z);
+                    } else {
+                        hb |= bit[u];
+                    }
+                } else {
+                    term(ent[u], pj[u], nj[u]);
+                }
+            }
+        }
+        // the general pairs among the hits
+        while (hb) {
+            const int k = __ffs(int(hb)) - 1;
+            hb &= hb - 1u;
+            const uint32_t ent = __ldg(shell - int64_t(k + k0) * 32);
+            const T4 pj = ldg4<R>(pos + (ent & NB_MASK)), nj = ldg4<R>(nrm + (ent & NB_MASK));
+            R d[3], ee = 0;
+            offset(ent, pj, d);
             R3<R> df = {0, 0, 0}, dt = {0, 0, 0};
-            if ((V & FORM_MERGED) && !__all_sync(__activemask(), (ty | tj) == 0) && (ty == 0 || tj == 0) &&
-                F.pair[ty | tj].kind == PAIR_ANISO) {
-                // one anisotropic path for the warp, as in the uncompensated form
-                // below; a lipid-lipid pair is added only inside its range, a
-                // protein pair always (as the general path does)
-                const PairP<R> &P = F.pair[ty | tj];
-                const bool inr = r2 < P.cutsq && r2 > R(1e-5);
-                if (inr) aniso<R, E>(P, dx, dy, dz, r2, ni.x, ni.y, ni.z, nj.x, nj.y, nj.z, df, dt, e);
-                if (inr || (ty | tj) != 0) accumulate(df, dt);
-            } else if ((ty | tj) == 0) {
-                if (r2 < ll_cutsq && r2 > R(1e-5)) {
-                    aniso<R, E>(a.ll, dx, dy, dz, r2, ni.x, ni.y, ni.z, nj.x, nj.y, nj.z, df, dt, e);
-                    accumulate(df, dt);
-                }
-            } else {
-                pair_general<R, E, (V & FORM_INLINE) != 0>(F.pair[ty * NT + tj], dx, dy, dz, r2, ni.x, ni.y, ni.z,
-                                                           nj.x, nj.y, nj.z, df, dt, e);
-                accumulate(df, dt);
+            pair_general<R, E>(F.pair[ty * NT + w_type(wbits(pj.w))], d[0], d[1], d[2], dist2(d), ni.x, ni.y, ni.z,
+                               nj.x, nj.y, nj.z, df, dt, ee);
+            const R v[6] = {df.x, df.y, df.z, dt.x, dt.y, dt.z};
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                if (K)
+                    kahan_add(A.s[q], A.c[K ? q : 0], v[q]);
+                else
+                    A.s[q] = add_rn(A.s[q], v[q]);
             }
-        } else if ((V & FORM_MERGED) && !__all_sync(__activemask(), (ty | tj) == 0)) {
-            /* Some lane of the warp has a protein in this pair: every lipid-lipid
-             * and lipid-protein pair of the warp goes through the same
-             * anisotropic code with its own parameters (row ty | tj of the
-             * table: the protein's type, 0 for two lipids), so that the
-             * protein's lane does not run after the lipids' lanes.  The
-             * parameters are those of the other branches: the results are
-             * the same bit for bit. */
-            if ((ty == 0 || tj == 0) && F.pair[ty | tj].kind == PAIR_ANISO) {
-                const PairP<R> &P = F.pair[ty | tj];
-                if (r2 < P.cutsq && r2 > R(1e-5))
-                    aniso<R, E>(P, dx, dy, dz, r2, ni.x, ni.y, ni.z, nj.x, nj.y, nj.z, f, t, e);
-            } else {
-                pair_general<R, E, (V & FORM_INLINE) != 0>(F.pair[ty * NT + tj], dx, dy, dz, r2, ni.x, ni.y, ni.z,
-                                                           nj.x, nj.y, nj.z, f, t, e);
-            }
-        } else if ((ty | tj) == 0) {
-            if (r2 < ll_cutsq && r2 > R(1e-5))
-                aniso<R, E>(a.ll, dx, dy, dz, r2, ni.x, ni.y, ni.z, nj.x, nj.y, nj.z, f, t, e);
-        } else {
-            pair_general<R, E, (V & FORM_INLINE) != 0>(F.pair[ty * NT + tj], dx, dy, dz, r2, ni.x, ni.y, ni.z, nj.x,
-                                                       nj.y, nj.z, f, t, e);
+            if (E) A.e = add_rn(A.e, ee);
         }
-    };
-    // Shell rows: partners in the skin at the last build, mostly still outside
-    // the range; returns whether row k's partner has come inside it.
-    auto shell_hit = [&](int k, uint32_t &ent, T4 &pj) {
-        ent = __ldg(shell - int64_t(k) * stride);  // the rows were prefetched into L1 (read-only path)
-        pj = ldg4<R>(pos + int(ent & NB_MASK));
-        const T4 s = sh[ent >> NB_SHIFT];
-        const R dx = (pi.x - pj.x) + s.x;
-        const R dy = (pi.y - pj.y) + s.y;
-        const R dz = (pi.z - pj.z) + s.z;
-        const R r2 = dx * dx + dy * dy + dz * dz;
-        const int tj = w_type(wbits(pj.w));
-        const R lim = ((ty | tj) == 0) ? ll_cutsq : F.pair[ty * NT + tj].anysq;
-        return r2 < lim;
-    };
-    if (V & FORM_MERGED) {
-        /* shell rows first, distance only: row k's hit is bit k of hm (rows
-         * beyond 32 are evaluated on the spot, after the merged pass, as
-         * without this form) */
-        uint32_t hm = 0;
-        const int nq = min(nout, 32);
-        for (int k = 0; k < nq; ++k) {
-            uint32_t ent;
-            T4 pj;
-            if (shell_hit(k, ent, pj)) hm |= 1u << k;
-        }
-        // inner rows, then the shell hits in row order, in one loop
-        const int total = nin + __popc(hm);
-        auto entry = [&](int k) -> uint32_t {
-            if (k < nin) return __ldg(nb + int64_t(k) * stride);
-            const int b = __ffs(hm) - 1;
-            hm &= hm - 1u;
-            return __ldg(shell - int64_t(b) * stride);
-        };
-        uint32_t e1 = total > 0 ? entry(0) : 0u;
-        uint32_t e2 = total > 1 ? entry(1) : 0u;
-        T4 pn, nn;
-        if (total > 0) {
-            pn = ldg4<R>(pos + int(e1 & NB_MASK));
-            nn = ldg4<R>(nrm + int(e1 & NB_MASK));
-        }
-        for (int k = 0; k < total; ++k) {
-            const uint32_t ent = e1;
-            const T4 pj = pn, nj = nn;
-            e1 = e2;
-            if (k + 2 < total) e2 = entry(k + 2);
-            if (k + 1 < total) {
-                pn = ldg4<R>(pos + int(e1 & NB_MASK));
-                nn = ldg4<R>(nrm + int(e1 & NB_MASK));
-            }
-            pair(ent, pj, nj);
-        }
-        for (int k = 32; k < nout; ++k) {
-            uint32_t ent;
-            T4 pj;
-            if (shell_hit(k, ent, pj)) pair(ent, pj, ldg4<R>(nrm + int(ent & NB_MASK)));
-        }
-    } else {
-        // Inner rows: partners that were inside the interaction range at the last
-        // build; almost all still are, so every lane does the pair arithmetic.
-        if (V & FORM_PIPE) {
-            /* software-pipelined: the entry two ahead and the gathers one ahead
-             * are in flight while the current pair is evaluated */
-            uint32_t e1 = nin > 0 ? __ldcs(nb) : 0u;
-            uint32_t e2 = nin > 1 ? __ldcs(nb + stride) : 0u;
-            T4 pn, nn;
-            if (nin > 0) {
-                pn = ldg4<R>(pos + int(e1 & NB_MASK));
-                nn = ldg4<R>(nrm + int(e1 & NB_MASK));
-            }
-            for (int k = 0; k < nin; ++k) {
-                const uint32_t ent = e1;
-                const T4 pj = pn, nj = nn;
-                e1 = e2;
-                if (k + 2 < nin) e2 = __ldcs(nb + int64_t(k + 2) * stride);
-                if (k + 1 < nin) {
-                    pn = ldg4<R>(pos + int(e1 & NB_MASK));
-                    nn = ldg4<R>(nrm + int(e1 & NB_MASK));
-                }
-                pair(ent, pj, nj);
-            }
-        } else {
-#pragma unroll 2
-            for (int k = 0; k < nin; ++k) {
-                const uint32_t ent = __ldcs(nb + int64_t(k) * stride);
-                const int j = int(ent & NB_MASK);
-                pair(ent, ldg4<R>(pos + j), ldg4<R>(nrm + j));
-            }
-        }
-        // the orientation is only gathered for the few shell partners that came in
-#pragma unroll 2
-        for (int k = 0; k < nout; ++k) {
-            uint32_t ent;
-            T4 pj;
-            if (shell_hit(k, ent, pj)) pair(ent, pj, ldg4<R>(nrm + int(ent & NB_MASK)));
-        }
+        if (!__any_sync(0xffffffffu, nout > k0 + 32)) break;
+        nin = kmin = 0;
     }
-    // bonds
-    const int bd = w_bdeg(w);
-    if (bd) {
-        const int ci = a.cell[lp][i];
+}
+
+/* Force of bond b and of face b on the vertex in slot i. */
+template<class R, bool E>
+__device__ __forceinline__ R3<R> bond_force(const KArgs<R> &a, const FFDev<R> &F, int i, int b, int lp,
+                                            const typename Vec<R>::T4 *__restrict__ pos,
+                                            const typename Vec<R>::T4 &pi, int ci, const SysDev &sd, R &e, int &flags) {
+    const BondSlot bs = a.bond[lp][int64_t(b) * a.npad + i];
+    const typename Vec<R>::T4 pj = pos[bs.partner];
+    R dx, dy, dz;
+    rel_pos<R>(sd, a.cell[lp][bs.partner], ci, pj, pi, dx, dy, dz);
+    const R r = sqrt(dx * dx + dy * dy + dz * dz);
+    const R kap = bond_kappa<R, E>(F.bond[bs.type], R(bs.r0), r, e, flags);
+    return {kap * dx, kap * dy, kap * dz};
+}
+template<class R>
+__device__ __forceinline__ R3<R> face_force(const KArgs<R> &a, int i, int b, int lp,
+                                            const typename Vec<R>::T4 *__restrict__ pos,
+                                            const typename Vec<R>::T4 &pi, int ci, const SysDev &sd, R cv, R ca) {
+    const int2 fs = a.fslot[lp][int64_t(b) * a.npad + i];
+    R bx, by, bz, cx, cy, cz;
+    rel_pos<R>(sd, a.cell[lp][fs.x], ci, pos[fs.x], pi, bx, by, bz);
+    rel_pos<R>(sd, a.cell[lp][fs.y], ci, pos[fs.y], pi, cx, cy, cz);
+    const R nx = by * cz - bz * cy, ny = bz * cx - bx * cz, nz = bx * cy - by * cx;  // 6 dV/da
+    const R inn = rnorm3(nx, ny, nz);
+    const R hx = nx * inn, hy = ny * inn, hz = nz * inn;
+    const R ex = bx - cx, ey = by - cy, ez = bz - cz;
+    const R gx = ey * hz - ez * hy, gy = ez * hx - ex * hz, gz = ex * hy - ey * hx;  // 2 dA/da
+    return {cv * nx + ca * gx, cv * ny + ca * gy, cv * nz + ca * gz};
+}
+
+/* Bonds and the mesh constraint of slot i, added to f in order.  A membrane
+ * has few vertices (0.8 % of the 4M-particle cell), each with about six bonds
+ * and six faces, so a warp's one or two vertices would walk a dozen dependent
+ * gathers alone: where a warp holds fewer vertices than its longest walk, its
+ * lanes take one bond or face each of one vertex after the other, and the
+ * owner adds their forces in the same order.  All 32 lanes must call it. */
+template<class R, bool E, bool K>
+__device__ __forceinline__ void bond_mesh_forces(const KArgs<R> &a, const FFDev<R> &F, int i, int cur, int lp, int w,
+                                                 const typename Vec<R>::T4 &pi, const SysDev &sd, const SysState &ss,
+                                                 R3<R> &f, R &e, int &flags) {
+    using T4 = typename Vec<R>::T4;
+    const bool real = w_type(w) != GHOST;
+    const int bd = real ? w_bdeg(w) : 0;
+    int fd = real ? w_fdeg(w) : 0;
+    if (!__any_sync(0xffffffffu, (bd | fd) != 0)) return;
+    const R cv = R(ss.cv) * R(1.0 / 6.0), ca = R(ss.ca) * R(0.5);
+    if (ss.cv == 0.0 && ss.ca == 0.0) fd = 0;
+    const T4 *__restrict__ pos = a.pos[cur];
+    const int ci = bd + fd > 0 ? a.cell[lp][i] : 0;
+    R3<R> c = {0, 0, 0};
+    auto accumulate = [&](const R3<R> &d) {
+        if (K) {
+            kahan_add(f.x, c.x, d.x);
+            kahan_add(f.y, c.y, d.y);
+            kahan_add(f.z, c.z, d.z);
+        } else {
+            f.x += d.x;
+            f.y += d.y;
+            f.z += d.z;
+        }
+    };
+    unsigned todo = __ballot_sync(0xffffffffu, bd + fd > 0);
+    if (__popc(todo) >= int(__reduce_max_sync(0xffffffffu, unsigned(bd + fd)))) {
         for (int b = 0; b < bd; ++b) {
-            const BondSlot bs = a.bond[lp][int64_t(b) * a.npad + i];
-            const T4 pj = pos[bs.partner];
-            R dx, dy, dz;
-            rel_pos<R>(sd, a.cell[lp][bs.partner], ci, pj, pi, dx, dy, dz);
-            const R r = sqrt(dx * dx + dy * dy + dz * dz);
-            const R kap = bond_kappa<R, E>(F.bond[bs.type], R(bs.r0), r, e, flags);
-            if (KAHAN) {
-                kahan_add(f.x, cf.x, kap * dx);
-                kahan_add(f.y, cf.y, kap * dy);
-                kahan_add(f.z, cf.z, kap * dz);
-            } else {
-                f.x += kap * dx;
-                f.y += kap * dy;
-                f.z += kap * dz;
+            R eb = 0;
+            accumulate(bond_force<R, E>(a, F, i, b, lp, pos, pi, ci, sd, eb, flags));
+            if (E) e += eb;
+        }
+        for (int b = 0; b < fd; ++b) accumulate(face_force<R>(a, i, b, lp, pos, pi, ci, sd, cv, ca));
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    while (todo) {
+        const int o = __ffs(int(todo)) - 1;
+        todo &= todo - 1u;
+        const int obd = __shfl_sync(0xffffffffu, bd, o), ofd = __shfl_sync(0xffffffffu, fd, o);
+        const int oi = __shfl_sync(0xffffffffu, i, o), oci = __shfl_sync(0xffffffffu, ci, o);
+        T4 op = pi;
+        op.x = __shfl_sync(0xffffffffu, pi.x, o);
+        op.y = __shfl_sync(0xffffffffu, pi.y, o);
+        op.z = __shfl_sync(0xffffffffu, pi.z, o);
+        R3<R> d = {0, 0, 0};
+        R eb = 0;
+        if (lane < obd)
+            d = bond_force<R, E>(a, F, oi, lane, lp, pos, op, oci, sd, eb, flags);
+        else if (lane < obd + ofd)
+            d = face_force<R>(a, oi, lane - obd, lp, pos, op, oci, sd, cv, ca);
+        for (int b = 0; b < obd + ofd; ++b) {
+            const R3<R> db = {__shfl_sync(0xffffffffu, d.x, b), __shfl_sync(0xffffffffu, d.y, b),
+                              __shfl_sync(0xffffffffu, d.z, b)};
+            const R ee = E ? __shfl_sync(0xffffffffu, eb, b) : R(0);
+            if (lane == o) {
+                accumulate(db);
+                if (E && b < obd) e += ee;
             }
         }
     }
-    // global area / volume constraint on mesh vertices
-    const int fd = w_fdeg(w);
-    if (fd && (ss.cv != 0.0 || ss.ca != 0.0)) {
-        const int ci = a.cell[lp][i];
-        const R cv = R(ss.cv) * R(1.0 / 6.0), ca = R(ss.ca) * R(0.5);
-        for (int b = 0; b < fd; ++b) {
-            const int2 fs = a.fslot[lp][int64_t(b) * a.npad + i];
-            R bx, by, bz, cx, cy, cz;
-            rel_pos<R>(sd, a.cell[lp][fs.x], ci, pos[fs.x], pi, bx, by, bz);
-            rel_pos<R>(sd, a.cell[lp][fs.y], ci, pos[fs.y], pi, cx, cy, cz);
-            const R nx = by * cz - bz * cy, ny = bz * cx - bx * cz, nz = bx * cy - by * cx;  // 6 dV/da
-            const R inn = rnorm3(nx, ny, nz);
-            const R hx = nx * inn, hy = ny * inn, hz = nz * inn;
-            const R ex = bx - cx, ey = by - cy, ez = bz - cz;
-            const R gx = ey * hz - ez * hy, gy = ez * hx - ex * hz, gz = ex * hy - ey * hx;  // 2 dA/da
-            if (KAHAN) {
-                kahan_add(f.x, cf.x, cv * nx + ca * gx);
-                kahan_add(f.y, cf.y, cv * ny + ca * gy);
-                kahan_add(f.z, cf.z, cv * nz + ca * gz);
-            } else {
-                f.x += cv * nx + ca * gx;
-                f.y += cv * ny + ca * gy;
-                f.z += cv * nz + ca * gz;
-            }
-        }
+}
+
+/* All forces and torques on slot i (all 32 lanes of the warp must call it; a
+ * ghost's are zero). */
+template<class R, bool E, bool K, int U>
+__device__ __forceinline__ void slot_forces(const KArgs<R> &a, const FFDev<R> &F, int i, int cur, int lp, int w,
+                                            const typename Vec<R>::T4 &pi, const typename Vec<R>::T4 &ni,
+                                            const SysDev &sd, const SysState &ss, int packed,
+                                            const ShiftTab<R> &sh, R3<R> &f, R3<R> &t, R &e, int &flags) {
+    const bool real = w_type(w) != GHOST;
+    const int ty = real ? w_type(w) : 0;
+    const PairP<R> &pl = F.pair[ty * NT];  // with a lipid
+    const OwnP<R> P = own_params(pl);
+    PairAcc<R, K> A;
+    A.clear();
+    const R lim = F.reach2[ty];
+    const int own_gen = pl.kind == PAIR_ANISO ? 0 : 1;
+    pair_sums<R, E, K, U>(a, F, P, lim, own_gen, i, a.pos[cur], a.nrm[cur], ty, packed, pi, ni, sh, A);
+    if (K) {
+#pragma unroll
+        for (int k = 0; k < NACC; ++k) A.s[k] = add_rn(A.s[k], -A.c[K ? k : 0]);
     }
+    f.x = fma_rn(A.s[6], ni.x, A.s[0]);
+    f.y = fma_rn(A.s[6], ni.y, A.s[1]);
+    f.z = fma_rn(A.s[6], ni.z, A.s[2]);
+    t.x = A.s[3];
+    t.y = A.s[4];
+    t.z = A.s[5];
+    e = A.e;
+    bond_mesh_forces<R, E, K>(a, F, i, cur, lp, w, pi, sd, ss, f, e, flags);
 }
 
 __device__ __forceinline__ void philox4(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t k0, uint32_t k1,
@@ -725,23 +819,18 @@ template<class R> __global__ void __launch_bounds__(RED_GROUP) k_reduce(KArgs<R>
     }
 }
 
-/* One particle of the fused Langevin step: forces at the current state, then
+/* One particle of the fused Langevin step, given its forces and torques:
  * src/integrate_langevin.h:105-146 (rotation, then translation with the
  * counter-based noise).  Writes the new state; returns the squared
- * displacement since the list was built, sum m v^2, the energy and the lipid
- * velocity (for the bulk-velocity removal). */
-template<class R, bool E, int V>
-__device__ __forceinline__ void langevin_particle(const KArgs<R> &a, const FFDev<R> &F, const typename Vec<R>::T4 *sh,
-                                                  int i, int s, int cur, int lp, long long step,
-                                                  const typename Vec<R>::T4 &pi, int w, bool zero_bulk, R &ke, R &ep,
-                                                  float &md2, int &flags, R &vsx, R &vsy, R &vsz) {
+ * displacement since the list was built, sum m v^2 and the lipid velocity
+ * (for the bulk-velocity removal). */
+template<class R>
+__device__ __forceinline__ void langevin_particle(const KArgs<R> &a, const FFDev<R> &F, int i, int s, int cur, int lp,
+                                                  long long step, const typename Vec<R>::T4 &pi,
+                                                  const typename Vec<R>::T4 &ni, int ty, bool zero_bulk, R3<R> f,
+                                                  const R3<R> &t, R &ke, float &md2, int &flags, R &vsx, R &vsy,
+                                                  R &vsz) {
     using T4 = typename Vec<R>::T4;
-    const int ty = w_type(w);
-    const SysDev &sd = a.sys[s];
-    const T4 ni = a.nrm[cur][i];
-    R3<R> f = {0, 0, 0}, t = {0, 0, 0};
-    R e = 0;
-    particle_forces<R, E, V>(a, F, i, cur, lp, w, pi, ni, sd, a.ss[s], sh, f, t, e, flags);
     const R dt = R(a.dt);
     T4 v = ldcs4<R>(&a.vel[lp][i]), o = ldcs4<R>(&a.omg[lp][i]);
     if (zero_bulk && ty == 0) {  // zero_bulk_velocity on the lipids (src/zero_bulk_velocity.h:38-45)
@@ -787,7 +876,6 @@ __device__ __forceinline__ void langevin_particle(const KArgs<R> &a, const FFDev
     md2 = float(ddx * ddx + ddy * ddy + ddz * ddz);
     if (!isfinite(p.x + p.y + p.z + v.x + v.y + v.z)) flags |= ERRB_NAN;
     ke = F.mass[ty] * (v.x * v.x + v.y * v.y + v.z * v.z);
-    ep = e;
     if (ty == 0) {
         vsx = v.x;
         vsy = v.y;
@@ -796,32 +884,33 @@ __device__ __forceinline__ void langevin_particle(const KArgs<R> &a, const FFDev
 }
 
 /* Langevin step with the per-system sums (energy, bulk-velocity removal):
- * the structure of the lite kernel below (small blocks, force-field table
- * through the read-only path) plus warp partials, summed per system by
- * k_reduce after the kernel.  Resident blocks as for k_nh_final (20, 18 with
- * the merged shell pass, 16 with compensated sums): 0.82 against 0.92 ms per
- * step with the merged pass on the 4.03M cell, where 20 blocks spilled. */
-template<class R, bool E, int V>
-__global__ void __launch_bounds__(LITE_BS, fp_blocks<R>((V & FORM_KAHAN) ? 16 : ((V & FORM_MERGED) ? 18 : 20)))
-    k_step_langevin(KArgs<R> a) {
-    if (halted(a.S)) return;
+ * the structure of the lite kernel below plus warp partials, summed per
+ * system by k_reduce after the kernel. */
+template<class R, bool E, bool K, int U>
+__global__ void __launch_bounds__(LITE_BS, force_blocks<R, E || K, U>()) k_step_langevin(KArgs<R> a) {
     using T4 = typename Vec<R>::T4;
-    __shared__ T4 sh[27];
-    init_shift<R>(a, sh);
-    const FFDev<R> *__restrict__ Fp = a.ff;
-    const int cur = __ldcg(&a.S->cur), lp = __ldcg(&a.S->lp);
-    const long long step = __ldcg(&a.S->step);
+    __shared__ ShiftTab<R> shm[LITE_BS / 32];
     const int i = blockIdx.x * LITE_BS + threadIdx.x;
-    const int s = a.blk_sys[i / SYS_PAD];
-    const T4 pi = a.pos[cur][i];
-    prefetch_warp_list(a.nbr, i, a.cap, a.nnb[i]);
+    // the loads that depend on nothing, together
+    const int4 sc = __ldcg(reinterpret_cast<const int4 *>(a.S));  // cur, lp, rebuild, error
+    const int s = a.nsys > 1 ? a.blk_sys[i / SYS_PAD] : 0;
+    const int packed = a.nnb[i];
+    if (halted(sc)) return;
+    const int cur = sc.x, lp = sc.y;
+    const FFDev<R> &F = *a.ff;
+    prefetch_warp_list(a.nbr, i, a.cap, packed);
+    ShiftTab<R> &sh = shm[threadIdx.x >> 5];
+    init_shift<R>(a.sys[s], sh);
+    const T4 pi = a.pos[cur][i], ni = a.nrm[cur][i];
     const int w = wbits(pi.w);
     R ke = 0, ep = 0, vsx = 0, vsy = 0, vsz = 0;
     float md2 = 0.f;
     int flags = 0;
+    R3<R> f, t;
+    slot_forces<R, E, K, U>(a, F, i, cur, lp, w, pi, ni, a.sys[s], a.ss[s], packed, sh, f, t, ep, flags);
     if (w_type(w) != GHOST)
-        langevin_particle<R, E, V>(a, *Fp, sh, i, s, cur, lp, step, pi, w, a.zero_bulk != 0, ke, ep, md2, flags, vsx,
-                                   vsy, vsz);
+        langevin_particle<R>(a, F, i, s, cur, lp, __ldcg(&a.S->step), pi, ni, w_type(w), a.zero_bulk != 0, f, t, ke,
+                             md2, flags, vsx, vsy, vsz);
     warp_partials<R>(a, i, ke, ep, md2, flags, vsx, vsy, vsz);
 }
 
@@ -831,27 +920,31 @@ __global__ void __launch_bounds__(LITE_BS, fp_blocks<R>((V & FORM_KAHAN) ? 16 : 
  * particles moved more than skin/2 raises the rebuild flag itself, and
  * k_advance flips the buffers after the kernel.  The temperature is reduced on
  * demand (k_vcom). */
-template<class R, int V>
-__global__ void __launch_bounds__(LITE_BS, fp_blocks<R>((V & 4) ? ((V & FORM_MERGED) ? 18 : 20) : 16))
-    k_step_langevin_lite(KArgs<R> a) {
-    if (halted(a.S)) return;
+template<class R, bool K, int U>
+__global__ void __launch_bounds__(LITE_BS, force_blocks<R, K, U>()) k_step_langevin_lite(KArgs<R> a) {
     using T4 = typename Vec<R>::T4;
-    __shared__ T4 sh[27];
-    init_shift<R>(a, sh);
-    const FFDev<R> *__restrict__ Fp = a.ff;
-    const int cur = __ldcg(&a.S->cur), lp = __ldcg(&a.S->lp);
-    const long long step = __ldcg(&a.S->step);
+    __shared__ ShiftTab<R> shm[LITE_BS / 32];
     const int i = blockIdx.x * LITE_BS + threadIdx.x;
-    const int s = a.blk_sys[i / SYS_PAD];
-    const T4 pi = a.pos[cur][i];
-    prefetch_warp_list(a.nbr, i, a.cap, a.nnb[i]);
+    // the loads that depend on nothing, together
+    const int4 sc = __ldcg(reinterpret_cast<const int4 *>(a.S));  // cur, lp, rebuild, error
+    const int s = a.nsys > 1 ? a.blk_sys[i / SYS_PAD] : 0;
+    const int packed = a.nnb[i];
+    if (halted(sc)) return;
+    const int cur = sc.x, lp = sc.y;
+    const FFDev<R> &F = *a.ff;
+    prefetch_warp_list(a.nbr, i, a.cap, packed);
+    ShiftTab<R> &sh = shm[threadIdx.x >> 5];
+    init_shift<R>(a.sys[s], sh);
+    const T4 pi = a.pos[cur][i], ni = a.nrm[cur][i];
     const int w = wbits(pi.w);
     R ke = 0, ep = 0, vsx = 0, vsy = 0, vsz = 0;
     float md2 = 0.f;
     int flags = 0;
+    R3<R> f, t;
+    slot_forces<R, false, K, U>(a, F, i, cur, lp, w, pi, ni, a.sys[s], a.ss[s], packed, sh, f, t, ep, flags);
     if (w_type(w) != GHOST)
-        langevin_particle<R, false, V>(a, *Fp, sh, i, s, cur, lp, step, pi, w, false, ke, ep, md2, flags, vsx, vsy,
-                                       vsz);
+        langevin_particle<R>(a, F, i, s, cur, lp, __ldcg(&a.S->step), pi, ni, w_type(w), false, f, t, ke, md2, flags,
+                             vsx, vsy, vsz);
     const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(md2));  // md2 >= 0: bit order = value order
     const int fl = int(__reduce_or_sync(0xffffffffu, unsigned(flags)));
     if ((threadIdx.x & 31) == 0) {
@@ -878,31 +971,34 @@ __global__ void k_advance(Scalars *S, int rebuild_every, int count_step) {
  * steepest-descent move of :113-130 and bounce_back (:132).  Positions and
  * orientations ping-pong like the Langevin step; the step counter (the noise
  * key) does not advance. */
-template<class R, int V>
-__global__ void __launch_bounds__(LITE_BS, fp_blocks<R>((V & 2) ? 12 : 16))
+template<class R, int U>
+__global__ void __launch_bounds__(LITE_BS, force_blocks<R, false, U>())
     k_minimize(KArgs<R> a, double dr_opt, double dn_opt) {
-    if (halted(a.S)) return;
     using T4 = typename Vec<R>::T4;
-    __shared__ T4 sh[27];
-    init_shift<R>(a, sh);
-    const FFDev<R> *__restrict__ Fp = a.ff;
-    const int cur = __ldcg(&a.S->cur), lp = __ldcg(&a.S->lp);
+    __shared__ ShiftTab<R> shm[LITE_BS / 32];
     const int i = blockIdx.x * LITE_BS + threadIdx.x;
-    const int s = a.blk_sys[i / SYS_PAD];
+    // the loads that depend on nothing, together
+    const int4 sc = __ldcg(reinterpret_cast<const int4 *>(a.S));  // cur, lp, rebuild, error
+    const int s = a.nsys > 1 ? a.blk_sys[i / SYS_PAD] : 0;
+    const int packed = a.nnb[i];
+    if (halted(sc)) return;
+    const int cur = sc.x, lp = sc.y;
+    const FFDev<R> &F = *a.ff;
+    prefetch_warp_list(a.nbr, i, a.cap, packed);
+    ShiftTab<R> &sh = shm[threadIdx.x >> 5];
+    init_shift<R>(a.sys[s], sh);
     const SysDev &sd = a.sys[s];
-    const T4 pi = a.pos[cur][i];
-    prefetch_warp_list(a.nbr, i, a.cap, a.nnb[i]);
+    const T4 pi = a.pos[cur][i], ni = a.nrm[cur][i];
     const int w = wbits(pi.w);
     const int ty = w_type(w);
     float md2 = 0.f;
     int flags = 0;
+    R3<R> f, t;
+    R e = 0;
+    slot_forces<R, false, false, U>(a, F, i, cur, lp, w, pi, ni, sd, a.ss[s], packed, sh, f, t, e, flags);
     if (ty != GHOST) {
-        const T4 ni = a.nrm[cur][i];
-        R3<R> f = {0, 0, 0}, t = {0, 0, 0};
-        R e = 0;
-        particle_forces<R, false, V>(a, *Fp, i, cur, lp, w, pi, ni, sd, a.ss[s], sh, f, t, e, flags);
         const R tx = ni.y * t.z - ni.z * t.y, ty_ = ni.z * t.x - ni.x * t.z, tz = ni.x * t.y - ni.y * t.x;
-        const R m = Fp->mass[ty];
+        const R m = F.mass[ty];
         const R dxx = f.x / m, dxy = f.y / m, dxz = f.z / m;
         const R dnx = ty_ * ni.z - tz * ni.y, dny = tz * ni.x - tx * ni.z, dnz = tx * ni.y - ty_ * ni.x;
         const R ndx = sqrt(dxx * dxx + dxy * dxy + dxz * dxz), ndn = sqrt(dnx * dnx + dny * dny + dnz * dnz);
@@ -941,33 +1037,30 @@ __global__ void __launch_bounds__(LITE_BS, fp_blocks<R>((V & 2) ? 12 : 16))
 
 /* Nose-Hoover second half (post_toque_final_update, src/integrate_nh.h:237-273)
  * fused with the forces: the lite structure plus warp partials for the
- * kinetic-energy sum that k_reduce turns into the thermostat update.  The
- * resident blocks asked for fall with the registers a form needs (20 blocks
- * at 48 registers, 18 at 56 with the merged shell pass, 16 at 64 with
- * compensated sums), so that those two forms do not spill. */
-template<class R, bool E, int V>
-__global__ void __launch_bounds__(LITE_BS, fp_blocks<R>((V & FORM_KAHAN) ? 16 : ((V & FORM_MERGED) ? 18 : 20)))
-    k_nh_final(KArgs<R> a, int count_step) {
-    if (halted(a.S)) return;
+ * kinetic-energy sum that k_reduce turns into the thermostat update. */
+template<class R, bool E, bool K, int U>
+__global__ void __launch_bounds__(LITE_BS, force_blocks<R, E || K, U>()) k_nh_final(KArgs<R> a, int count_step) {
     using T4 = typename Vec<R>::T4;
-    __shared__ T4 sh[27];
-    init_shift<R>(a, sh);
-    const FFDev<R> &F = *a.ff;
-    const int cur = __ldcg(&a.S->cur), lp = __ldcg(&a.S->lp);
+    __shared__ ShiftTab<R> shm[LITE_BS / 32];
     const int i = blockIdx.x * LITE_BS + threadIdx.x;
-    const int s = a.blk_sys[i / SYS_PAD];
-    const SysDev &sd = a.sys[s];
-    const T4 pi = a.pos[cur][i];
-    prefetch_warp_list(a.nbr, i, a.cap, a.nnb[i]);
+    // the loads that depend on nothing, together
+    const int4 sc = __ldcg(reinterpret_cast<const int4 *>(a.S));  // cur, lp, rebuild, error
+    const int s = a.nsys > 1 ? a.blk_sys[i / SYS_PAD] : 0;
+    const int packed = a.nnb[i];
+    if (halted(sc)) return;
+    const int cur = sc.x, lp = sc.y;
+    const FFDev<R> &F = *a.ff;
+    prefetch_warp_list(a.nbr, i, a.cap, packed);
+    ShiftTab<R> &sh = shm[threadIdx.x >> 5];
+    init_shift<R>(a.sys[s], sh);
+    const T4 pi = a.pos[cur][i], ni = a.nrm[cur][i];
     const int w = wbits(pi.w);
     const int ty = w_type(w);
     R ke = 0, ep = 0;
     int flags = 0;
+    R3<R> f, t;
+    slot_forces<R, E, K, U>(a, F, i, cur, lp, w, pi, ni, a.sys[s], a.ss[s], packed, sh, f, t, ep, flags);
     if (ty != GHOST) {
-        const T4 ni = a.nrm[cur][i];
-        R3<R> f = {0, 0, 0}, t = {0, 0, 0};
-        R e = 0;
-        particle_forces<R, E, V>(a, F, i, cur, lp, w, pi, ni, sd, a.ss[s], sh, f, t, e, flags);
         const R dt = R(a.dt);
         const R zeta = R(__ldcg(&a.ss[s].zeta));
         const R im = F.inv_mass[ty];
@@ -997,7 +1090,6 @@ __global__ void __launch_bounds__(LITE_BS, fp_blocks<R>((V & FORM_KAHAN) ? 16 : 
         a.trq[lp][i] = tq;
         if (!isfinite(v.x + v.y + v.z)) flags |= ERRB_NAN;
         ke = F.mass[ty] * (v.x * v.x + v.y * v.y + v.z * v.z);
-        ep = e;
     }
     warp_partials<R>(a, i, ke, ep, 0.f, flags);
 }
@@ -1107,26 +1199,28 @@ template<class R> __global__ void __launch_bounds__(256) k_assign_temperature(KA
     a.vel[lp][i] = v;
 }
 
-template<class R, bool E, int V> __global__ void __launch_bounds__(LITE_BS, fp_blocks<R>(16)) k_forces(KArgs<R> a) {
-    if (halted(a.S)) return;
+template<class R, bool K, int U>
+__global__ void __launch_bounds__(LITE_BS, force_blocks<R, true, U>()) k_forces(KArgs<R> a) {
     using T4 = typename Vec<R>::T4;
-    __shared__ T4 sh[27];
-    init_shift<R>(a, sh);
-    const FFDev<R> &F = *a.ff;
-    const int cur = __ldcg(&a.S->cur), lp = __ldcg(&a.S->lp);
+    __shared__ ShiftTab<R> shm[LITE_BS / 32];
     const int i = blockIdx.x * LITE_BS + threadIdx.x;
-    const int s = a.blk_sys[i / SYS_PAD];
-    const SysDev &sd = a.sys[s];
-    const T4 pi = a.pos[cur][i];
-    prefetch_warp_list(a.nbr, i, a.cap, a.nnb[i]);
+    // the loads that depend on nothing, together
+    const int4 sc = __ldcg(reinterpret_cast<const int4 *>(a.S));  // cur, lp, rebuild, error
+    const int s = a.nsys > 1 ? a.blk_sys[i / SYS_PAD] : 0;
+    const int packed = a.nnb[i];
+    if (halted(sc)) return;
+    const int cur = sc.x, lp = sc.y;
+    const FFDev<R> &F = *a.ff;
+    prefetch_warp_list(a.nbr, i, a.cap, packed);
+    ShiftTab<R> &sh = shm[threadIdx.x >> 5];
+    init_shift<R>(a.sys[s], sh);
+    const T4 pi = a.pos[cur][i], ni = a.nrm[cur][i];
     const int w = wbits(pi.w);
-    R ep = 0;
     int flags = 0;
+    R3<R> f, t;
+    R e = 0;
+    slot_forces<R, true, K, U>(a, F, i, cur, lp, w, pi, ni, a.sys[s], a.ss[s], packed, sh, f, t, e, flags);
     if (w_type(w) != GHOST) {
-        const T4 ni = a.nrm[cur][i];
-        R3<R> f = {0, 0, 0}, t = {0, 0, 0};
-        R e = 0;
-        particle_forces<R, E, V>(a, F, i, cur, lp, w, pi, ni, sd, a.ss[s], sh, f, t, e, flags);
         T4 q = pi;
         q.x = f.x;
         q.y = f.y;
@@ -1137,9 +1231,10 @@ template<class R, bool E, int V> __global__ void __launch_bounds__(LITE_BS, fp_b
         q.z = t.z;
         a.trq[lp][i] = q;
         a.epart[i] = double(e);
-        ep = e;
+    } else {
+        e = 0;
     }
-    warp_partials<R>(a, i, R(0), ep, 0.f, flags);
+    warp_partials<R>(a, i, R(0), e, 0.f, flags);
 }
 
 /* FP64 membrane area and enclosed volume of each system's face mesh, and
@@ -1231,105 +1326,91 @@ template<class R> __global__ void __launch_bounds__(256) k_mesh(KArgs<R> a) {
 
 }  // namespace
 
-/* Force-kernel forms: the bits of FORM_* above (the list-build form, bits 3-4
- * of orbc_params.kernel_variant, is handled by the rebuild).  The merged and
- * compensated bits are instantiated on top of the pipelined, inlined loop. */
 template<class R> void reduce_sums(const KArgs<R> &a, int mode, int count_step, cudaStream_t st) {
     k_reduce<R><<<a.ngroups, RED_GROUP, 0, st>>>(a, mode, count_step);
 }
-/* the pair-loop bits of a form (FORM_OCC dropped), rounded to an instantiated one */
-constexpr int loop_form(int v) {
-    return (v & (FORM_MERGED | FORM_KAHAN)) ? ((v & (FORM_MERGED | FORM_KAHAN)) | FORM_PIPE | FORM_INLINE) : (v & 3);
-}
-template<class R, int V> void step_langevin_v(const KArgs<R> &a, cudaStream_t st, bool energy) {
-    if (energy) {
-        k_step_langevin<R, true, loop_form(V)><<<a.npad / LITE_BS, LITE_BS, 0, st>>>(a);
-        reduce_sums<R>(a, MODE_LANGEVIN, 1, st);
-    } else if (a.zero_bulk) {
-        k_step_langevin<R, false, loop_form(V)><<<a.npad / LITE_BS, LITE_BS, 0, st>>>(a);
-        reduce_sums<R>(a, MODE_LANGEVIN, 1, st);
-    } else {
-        k_step_langevin_lite<R, V><<<a.npad / LITE_BS, LITE_BS, 0, st>>>(a);
-        k_advance<<<1, 1, 0, st>>>(a.S, a.rebuild_every, 1);
-    }
-}
-template<class R, int V> void nh_final_v(const KArgs<R> &a, cudaStream_t st, bool energy) {
-    if (energy)
-        k_nh_final<R, true, V><<<a.npad / LITE_BS, LITE_BS, 0, st>>>(a, 1);
+/* launch(U, blocks) with the batch of rows that the size asks for.  FP32: four
+ * rows together while all blocks are resident at once (10 per SM, 152 SMs: up
+ * to 97 thousand slots), where the chain of dependent gathers sets the time
+ * and nothing else competes for the registers; beyond that two, whose 16
+ * resident blocks hide more than the longer batch does.  Step kernel, batches
+ * of two / four: 2,048 particles 18.8 / 15.4 us, 32,768: 20.9 / 18.3 us, 131,946:
+ * 29 / 34 us, 1.0M: 174 / 243 us.  FP64: one row (the FP64 pipe is the bound:
+ * 1.11 against 1.13 and 1.15 ms on a 250 thousand particle cell). */
+template<class R, class L> void by_batch(const KArgs<R> &a, L launch) {
+    const int nb = a.npad / LITE_BS;
+    if constexpr (sizeof(R) == 8)
+        launch(std::integral_constant<int, 1>(), nb);
+    else if (nb <= 152 * force_blocks<R, false, 4>())
+        launch(std::integral_constant<int, 4>(), nb);
     else
-        k_nh_final<R, false, V><<<a.npad / LITE_BS, LITE_BS, 0, st>>>(a, 1);
-    reduce_sums<R>(a, MODE_NH_FINAL, 1, st);
+        launch(std::integral_constant<int, 2>(), nb);
+}
+template<class R, bool K> void step_langevin_v(const KArgs<R> &a, cudaStream_t st, bool energy) {
+    by_batch<R>(a, [&](auto u, int nb) {
+        constexpr int U = decltype(u)::value;
+        if (energy)
+            k_step_langevin<R, true, K, U><<<nb, LITE_BS, 0, st>>>(a);
+        else if (a.zero_bulk)
+            k_step_langevin<R, false, K, U><<<nb, LITE_BS, 0, st>>>(a);
+        else
+            k_step_langevin_lite<R, K, U><<<nb, LITE_BS, 0, st>>>(a);
+    });
+    if (energy || a.zero_bulk)
+        reduce_sums<R>(a, MODE_LANGEVIN, 1, st);
+    else
+        k_advance<<<1, 1, 0, st>>>(a.S, a.rebuild_every, 1);
 }
 template<class R> void launch_step_langevin(const KArgs<R> &a, cudaStream_t st, bool energy) {
-    const int ext = a.variant & (FORM_MERGED | FORM_KAHAN);
-    if (ext) {  // the extended forms, with or without the occupancy form
-        const bool occ = (a.variant & FORM_OCC) != 0;
-        switch (ext | (occ ? FORM_OCC : 0)) {
-            case FORM_MERGED: step_langevin_v<R, FORM_MERGED | 3>(a, st, energy); break;
-            case FORM_KAHAN: step_langevin_v<R, FORM_KAHAN | 3>(a, st, energy); break;
-            case FORM_MERGED | FORM_KAHAN: step_langevin_v<R, FORM_MERGED | FORM_KAHAN | 3>(a, st, energy); break;
-            case FORM_MERGED | FORM_OCC: step_langevin_v<R, FORM_MERGED | 7>(a, st, energy); break;
-            case FORM_KAHAN | FORM_OCC: step_langevin_v<R, FORM_KAHAN | 7>(a, st, energy); break;
-            default: step_langevin_v<R, FORM_MERGED | FORM_KAHAN | 7>(a, st, energy); break;
-        }
-        return;
-    }
-    switch (a.variant & 7) {
-        case 1: step_langevin_v<R, 1>(a, st, energy); break;
-        case 2: step_langevin_v<R, 2>(a, st, energy); break;
-        case 3: step_langevin_v<R, 3>(a, st, energy); break;
-        case 4: step_langevin_v<R, 4>(a, st, energy); break;
-        case 5: step_langevin_v<R, 5>(a, st, energy); break;
-        case 6: step_langevin_v<R, 6>(a, st, energy); break;
-        case 7: step_langevin_v<R, 7>(a, st, energy); break;
-        default: step_langevin_v<R, 0>(a, st, energy); break;
-    }
+    if (a.kahan)
+        step_langevin_v<R, true>(a, st, energy);
+    else
+        step_langevin_v<R, false>(a, st, energy);
+}
+template<class R, bool K> void nh_final_v(const KArgs<R> &a, cudaStream_t st, bool energy, int count_step) {
+    by_batch<R>(a, [&](auto u, int nb) {
+        constexpr int U = decltype(u)::value;
+        if (energy)
+            k_nh_final<R, true, K, U><<<nb, LITE_BS, 0, st>>>(a, count_step);
+        else
+            k_nh_final<R, false, K, U><<<nb, LITE_BS, 0, st>>>(a, count_step);
+    });
+    reduce_sums<R>(a, MODE_NH_FINAL, count_step, st);
 }
 template<class R> void launch_nh_final(const KArgs<R> &a, cudaStream_t st, bool energy) {
-    switch (loop_form(a.variant)) {
-        case 1: nh_final_v<R, 1>(a, st, energy); break;
-        case 2: nh_final_v<R, 2>(a, st, energy); break;
-        case 3: nh_final_v<R, 3>(a, st, energy); break;
-        case FORM_MERGED | 3: nh_final_v<R, FORM_MERGED | 3>(a, st, energy); break;
-        case FORM_KAHAN | 3: nh_final_v<R, FORM_KAHAN | 3>(a, st, energy); break;
-        case FORM_MERGED | FORM_KAHAN | 3: nh_final_v<R, FORM_MERGED | FORM_KAHAN | 3>(a, st, energy); break;
-        default: nh_final_v<R, 0>(a, st, energy); break;
-    }
+    if (a.kahan)
+        nh_final_v<R, true>(a, st, energy, 1);
+    else
+        nh_final_v<R, false>(a, st, energy, 1);
 }
 template<class R> void launch_nh_prologue(const KArgs<R> &a, cudaStream_t st) {
-    if (a.variant & FORM_KAHAN)
-        k_nh_final<R, true, FORM_KAHAN | 3><<<a.npad / LITE_BS, LITE_BS, 0, st>>>(a, 0);
+    if (a.kahan)
+        nh_final_v<R, true>(a, st, true, 0);
     else
-        k_nh_final<R, true, 0><<<a.npad / LITE_BS, LITE_BS, 0, st>>>(a, 0);
-    reduce_sums<R>(a, MODE_NH_FINAL, 0, st);
+        nh_final_v<R, false>(a, st, true, 0);
 }
 template<class R> void launch_nh_initial(const KArgs<R> &a, cudaStream_t st) {
     k_nh_initial<R><<<a.npad / 256, 256, 0, st>>>(a);
     reduce_sums<R>(a, MODE_NH_INITIAL, 0, st);
 }
-/* The forces hook evaluates pairs in the form's accumulation (plain or
- * compensated); the loop structure does not change the sums' order. */
 template<class R> void launch_forces(const KArgs<R> &a, cudaStream_t st) {
-    if (a.variant & FORM_KAHAN)
-        k_forces<R, true, FORM_KAHAN | 3><<<a.npad / LITE_BS, LITE_BS, 0, st>>>(a);
-    else
-        k_forces<R, true, 0><<<a.npad / LITE_BS, LITE_BS, 0, st>>>(a);
+    by_batch<R>(a, [&](auto u, int nb) {
+        constexpr int U = decltype(u)::value;
+        if (a.kahan)
+            k_forces<R, true, U><<<nb, LITE_BS, 0, st>>>(a);
+        else
+            k_forces<R, false, U><<<nb, LITE_BS, 0, st>>>(a);
+    });
     reduce_sums<R>(a, MODE_FORCES, 0, st);
 }
 template<class R> void launch_mesh(const KArgs<R> &a, cudaStream_t st) {
     if (a.nmblk > 0) k_mesh<R><<<a.nmblk, 256, 0, st>>>(a);
 }
-template<class R, int V> void minimize_v(const KArgs<R> &a, double dr_opt, double dn_opt, cudaStream_t st) {
-    k_minimize<R, V><<<a.npad / LITE_BS, LITE_BS, 0, st>>>(a, dr_opt, dn_opt);
-    k_advance<<<1, 1, 0, st>>>(a.S, a.rebuild_every, 0);
-}
 template<class R> void launch_minimize(const KArgs<R> &a, double dr_opt, double dn_opt, cudaStream_t st) {
-    switch (a.variant & 3) {
-        case 1: minimize_v<R, 1>(a, dr_opt, dn_opt, st); break;
-        case 2: minimize_v<R, 2>(a, dr_opt, dn_opt, st); break;
-        case 3: minimize_v<R, 3>(a, dr_opt, dn_opt, st); break;
-        default: minimize_v<R, 0>(a, dr_opt, dn_opt, st); break;
-    }
+    by_batch<R>(a, [&](auto u, int nb) {
+        k_minimize<R, decltype(u)::value><<<nb, LITE_BS, 0, st>>>(a, dr_opt, dn_opt);
+    });
+    k_advance<<<1, 1, 0, st>>>(a.S, a.rebuild_every, 0);
 }
 template<class R> void launch_vcom(const KArgs<R> &a, cudaStream_t st) {
     k_vcom<R><<<a.npad / 256, 256, 0, st>>>(a);
