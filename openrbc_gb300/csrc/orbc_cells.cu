@@ -7,10 +7,12 @@
 // Rebuild chain (runs only when a particle moved more than skin/2 since the
 // last build, or on demand):
 //   k_rebin          re-express each position in the cell that now holds it,
-//                    clear the old cell ranges, emit (cell key, slot) pairs
-//   LSD radix sort   stable, 8-bit digits, (key, slot) -> sorted + inverse map
-//   k_ranges_gather  cell [begin, end) ranges and the physical reorder of all
-//                    per-particle arrays (bond / face partners remapped)
+//                    clear the old cell ranges, count cells and tiles
+//   k_tile_scan      prefix of the particles per tile of 64 cells
+//   k_tile_cells     [begin, end) of each occupied cell
+//   k_place, k_rank  slots by cell, in the order of their old slots
+//   k_gather         the physical reorder of all per-particle arrays (bond /
+//                    face partners remapped)
 //   k_nlist          full neighbour list per particle from the 27 cells
 //                    around its own; the last block flips buffer parities
 #include "orbc_device.cuh"
@@ -173,6 +175,11 @@ int radix_sort_pairs(uint32_t *keys[2], int *vals[2], int *counts, int *digit_to
 /* ------------------------------------------------------------------------- */
 /* Rebuild chain                                                             */
 /* ------------------------------------------------------------------------- */
+/* The particles are ordered by (cell id, old slot) without sorting keys: cells
+ * are counted, tiles of 64 cells are scanned, and the handful of particles of a
+ * cell are ranked by their old slot.  An LSD radix sort of the ids (three or
+ * four passes of three kernels) took 58 us for 33 thousand particles and 190 us for
+ * 4.0M, most of it launches and serial scans. */
 template<class R> __global__ void __launch_bounds__(256) k_rebin(KArgs<R> a, int gated) {
     using T4 = typename Vec<R>::T4;
     if (gated && !__ldcg(&a.S->rebuild)) return;
@@ -182,64 +189,191 @@ template<class R> __global__ void __launch_bounds__(256) k_rebin(KArgs<R> a, int
         a.S->out_of_grid = 0;
     }
     int out = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.npad; i += gridDim.x * blockDim.x) {
-        const SysDev &sd = a.sys[a.blk_sys[i / SYS_PAD]];
-        T4 p = a.pos[cur][i];
-        const int w = wbits(p.w);
-        uint32_t key;
-        if (w_type(w) == GHOST) {
-            key = sd.cell_base + ncell_ids(sd);
-        } else {
-            const int c = a.cell[lp][i];
-            int cc[3] = {cx_of(c), cy_of(c), cz_of(c)};
-            a.ranges[sd.cell_base + cell_code(sd, cc[0], cc[1], cc[2])] = make_int2(0, 0);
-            R o[3] = {p.x, p.y, p.z};
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;  // npad is a multiple of the block size
+    const int s = a.blk_sys[i / SYS_PAD];
+    const SysDev &sd = a.sys[s];
+    T4 p = a.pos[cur][i];
+    const bool real = w_type(wbits(p.w)) != GHOST;
+    uint32_t key = 0xffffffffu;
+    if (real) {
+        const int c = a.cell[lp][i];
+        int cc[3] = {cx_of(c), cy_of(c), cz_of(c)};
+        a.ranges[sd.cell_base + cell_code(sd, cc[0], cc[1], cc[2])] = make_int2(0, 0);
+        R o[3] = {p.x, p.y, p.z};
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const R L = lc_of<R>(sd, d);
-                const R invL = inv_lc_of<R>(sd, d);
-                const int k = int(floor(add_rn(mul_rn(o[d], invL), R(0.5))));
-                int nc = cc[d] + k;
-                if (sd.per[d]) {
-                    o[d] = sub_rn(o[d], mul_rn(R(k), L));
-                    nc %= sd.nc[d];
-                    if (nc < 0) nc += sd.nc[d];
-                } else {
-                    const int cl = min(max(nc, 0), sd.nc[d] - 1);
-                    if (cl != nc) out = 1;
-                    o[d] = sub_rn(o[d], mul_rn(R(cl - cc[d]), L));
-                    nc = cl;
-                }
-                cc[d] = nc;
+        for (int d = 0; d < 3; ++d) {
+            const R L = lc_of<R>(sd, d);
+            const R invL = inv_lc_of<R>(sd, d);
+            const int k = int(floor(add_rn(mul_rn(o[d], invL), R(0.5))));
+            int nc = cc[d] + k;
+            if (sd.per[d]) {
+                o[d] = sub_rn(o[d], mul_rn(R(k), L));
+                nc %= sd.nc[d];
+                if (nc < 0) nc += sd.nc[d];
+            } else {
+                const int cl = min(max(nc, 0), sd.nc[d] - 1);
+                if (cl != nc) out = 1;
+                o[d] = sub_rn(o[d], mul_rn(R(cl - cc[d]), L));
+                nc = cl;
             }
-            p.x = o[0];
-            p.y = o[1];
-            p.z = o[2];
-            a.pos[cur][i] = p;  // the gather that follows sets the displacement reference
-            a.cell[lp][i] = cpack(cc[0], cc[1], cc[2]);
-            key = sd.cell_base + cell_code(sd, cc[0], cc[1], cc[2]);
+            cc[d] = nc;
         }
-        a.skey[0][i] = key;
-        a.sval[0][i] = i;
+        p.x = o[0];
+        p.y = o[1];
+        p.z = o[2];
+        a.pos[cur][i] = p;  // the gather that follows sets the displacement reference
+        a.cell[lp][i] = cpack(cc[0], cc[1], cc[2]);
+        key = sd.cell_base + cell_code(sd, cc[0], cc[1], cc[2]);
     }
+    a.skey[0][i] = key;
+    // one atomic per cell and per tile of the warp (its particles sit in a few
+    // cells); ghosts take the places behind the system's particles
+    const int lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    const int leader = __ffs(int(peers)) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(real ? a.ccnt + key : a.gcnt + s, __popc(peers));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    a.sval[1][i] = base + __popc(peers & ((1u << lane) - 1u));
+    const unsigned tpeers = __match_any_sync(0xffffffffu, key >> 6);
+    if (real && lane == __ffs(int(tpeers)) - 1) atomicAdd(a.tcnt + (key >> 6), __popc(tpeers));
     if (out) {
         atomicOr(&a.S->error, ERRB_GRID);
         atomicAdd(&a.S->out_of_grid, 1);
     }
 }
 
-template<class R> __global__ void __launch_bounds__(256) k_ranges_gather(KArgs<R> a, int fin, int gated) {
+/* Exclusive prefix of the tiles' particle counts inside each block of
+ * SCAN_TILES; the last block to finish turns the block totals into prefixes. */
+__global__ void __launch_bounds__(1024) k_tile_scan(const int *tcnt, int *tstart, int *bsum, int nscan,
+                                                    unsigned int *counter, const int *gate) {
+    if (gate_closed(gate)) return;
+    __shared__ int wsum[32];
+    __shared__ bool last;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    // inclusive prefix of v over the block; total in wsum[31]
+    auto scan = [&](int v) {
+        int x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            int w = wsum[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += y;
+            }
+            wsum[lane] = w;
+        }
+        __syncthreads();
+        return x + (warp > 0 ? wsum[warp - 1] : 0);
+    };
+    const int64_t q = int64_t(blockIdx.x) * (SCAN_TILES / 4) + t;
+    const int4 c = reinterpret_cast<const int4 *>(tcnt)[q];
+    const int sum = c.x + c.y + c.z + c.w;
+    const int e = scan(sum) - sum;
+    reinterpret_cast<int4 *>(tstart)[q] = make_int4(e, e + c.x, e + c.x + c.y, e + c.x + c.y + c.z);
+    if (t == 0) {
+        bsum[blockIdx.x] = wsum[31];
+        __threadfence();
+        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    int carry = 0;
+    for (int b0 = 0; b0 < nscan; b0 += 1024) {
+        const int v = b0 + t < nscan ? __ldcg(bsum + b0 + t) : 0;
+        const int x = scan(v);
+        if (b0 + t < nscan) bsum[b0 + t] = carry + x - v;
+        carry += wsum[31];
+        __syncthreads();  // wsum is read by all before the next scan
+    }
+    if (t == 0) *counter = 0;
+}
+
+/* Ranges of the occupied cells, one warp per 32 tiles; the counts go back to
+ * zero. */
+template<class R> __global__ void __launch_bounds__(256) k_tile_cells(KArgs<R> a, int gated) {
+    if (gated && !__ldcg(&a.S->rebuild)) return;
+    const int lane = threadIdx.x & 31;
+    const int t0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 32;
+    if (t0 >= a.nctile) return;
+    if (blockIdx.x == 0)
+        for (int s = threadIdx.x; s < a.nsys; s += blockDim.x) a.gcnt[s] = 0;
+    const int n = a.tcnt[t0 + lane];  // nctile is a multiple of 32
+    const int start = n ? a.tstart[t0 + lane] + a.bsum[(t0 + lane) / SCAN_TILES] : 0;
+    if (n) a.tcnt[t0 + lane] = 0;
+    for (unsigned m = __ballot_sync(0xffffffffu, n != 0); m; m &= m - 1u) {
+        const int l = __ffs(int(m)) - 1;
+        const int64_t id0 = int64_t(t0 + l) * 64;
+        int lo = 0, hi = a.nsys - 1;  // the system whose ids these are
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if (int64_t(a.sys[mid].cell_base) <= id0)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        const int base = __shfl_sync(0xffffffffu, start, l) + a.sys[lo].slot_shift;
+        const int c0 = a.ccnt[id0 + 2 * lane], c1 = a.ccnt[id0 + 2 * lane + 1];
+        int x = c0 + c1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        const int b = base + x - c0 - c1;
+        if (c0) {
+            a.ranges[id0 + 2 * lane] = make_int2(b, b + c0);
+            a.ccnt[id0 + 2 * lane] = 0;
+        }
+        if (c1) {
+            a.ranges[id0 + 2 * lane + 1] = make_int2(b + c0, b + c0 + c1);
+            a.ccnt[id0 + 2 * lane + 1] = 0;
+        }
+    }
+}
+
+/* Slots by cell in arrival order, then each slot's place by its rank among
+ * the old slots of its cell. */
+template<class R> __global__ void __launch_bounds__(256) k_place(KArgs<R> a, int gated) {
+    if (gated && !__ldcg(&a.S->rebuild)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t key = a.skey[0][i];
+    if (key != 0xffffffffu) a.skey[1][a.ranges[key].x + a.sval[1][i]] = uint32_t(i);
+}
+template<class R> __global__ void __launch_bounds__(256) k_rank(KArgs<R> a, int gated) {
+    if (gated && !__ldcg(&a.S->rebuild)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t key = a.skey[0][i];
+    int p;
+    if (key == 0xffffffffu) {
+        const SysDev &sd = a.sys[a.blk_sys[i / SYS_PAD]];
+        p = sd.off + sd.nreal + a.sval[1][i];
+    } else {
+        const int2 rg = a.ranges[key];
+        p = rg.x;
+        for (int q = rg.x; q < rg.y; ++q) p += a.skey[1][q] < uint32_t(i) ? 1 : 0;
+    }
+    a.sval[0][p] = i;
+    a.inv[i] = p;
+}
+
+template<class R> __global__ void __launch_bounds__(256) k_gather(KArgs<R> a, int gated) {
     if (gated && !__ldcg(&a.S->rebuild)) return;
     const int cur = __ldcg(&a.S->cur), lp = __ldcg(&a.S->lp);
     const int nc = 1 - cur, nl = 1 - lp;
-    const uint32_t *sk = a.skey[fin];
-    const int *sv = a.sval[fin];
+    const int *sv = a.sval[0];
     const int n = a.npad;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         // every load of the slot before its first store: the stores may alias
         // the loads as far as the compiler knows, and would serialise them
-        const uint32_t k = sk[p];
-        const bool first = p == 0 || sk[p - 1] != k, last = p == n - 1 || sk[p + 1] != k;
         const int src = sv[p];
         const auto ps = a.pos[cur][src];
         const auto ns = a.nrm[cur][src];
@@ -251,8 +385,6 @@ template<class R> __global__ void __launch_bounds__(256) k_ranges_gather(KArgs<R
             a.frc[nl][p] = fs;
             a.trq[nl][p] = qs;
         }
-        if (first) a.ranges[k].x = p;
-        if (last) a.ranges[k].y = p + 1;
         a.pos[nc][p] = ps;
         a.nrm[nc][p] = ns;
         a.vel[nl][p] = vs;
@@ -776,14 +908,17 @@ template<class R> void launch_rebuild_stage(const KArgs<R> &a, cudaStream_t st, 
     const int g = grid_for(a.npad);
     switch (stage) {
         case 0:
-            k_rebin<R><<<(a.npad + 255) / 256, 256, 0, st>>>(a, gated ? 1 : 0);
+            k_rebin<R><<<a.npad / 256, 256, 0, st>>>(a, gated ? 1 : 0);
             break;
         case 1:
-            radix_sort_pairs(const_cast<uint32_t **>(a.skey), const_cast<int **>(a.sval), a.counts, a.digit_total,
-                             a.inv, a.npad, a.sort_passes, a.ntiles, gated ? &a.S->rebuild : nullptr, st);
+            k_tile_scan<<<a.nscan, 1024, 0, st>>>(a.tcnt, a.tstart, a.bsum, a.nscan, &a.S->scan_counter,
+                                                  gated ? &a.S->rebuild : nullptr);
+            k_tile_cells<R><<<a.nctile / 256, 256, 0, st>>>(a, gated ? 1 : 0);
+            k_place<R><<<a.npad / 256, 256, 0, st>>>(a, gated ? 1 : 0);
+            k_rank<R><<<a.npad / 256, 256, 0, st>>>(a, gated ? 1 : 0);
             break;
         case 2:
-            k_ranges_gather<R><<<g, 256, 0, st>>>(a, a.sort_passes % 2, gated ? 1 : 0);
+            k_gather<R><<<g, 256, 0, st>>>(a, gated ? 1 : 0);
             break;
         default:
             if (a.nlist_lane == 2)

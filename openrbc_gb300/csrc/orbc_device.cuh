@@ -109,8 +109,9 @@ struct SysDev {
     double wlo[3], whi[3];          // reflective walls (Nose-Hoover bounce-back)
     int nc[3], per[3];
     int ntile[3], pad0;             // 4 x 4 x 4 tiles of cells per axis (cell-id order)
-    unsigned cell_base;             // first global cell id; ncell + 1 ids (last = ghost cell)
+    unsigned cell_base;             // first global cell id (a multiple of 64: whole tiles)
     int off, npad, nreal;
+    int slot_shift;                 // off - particles of the systems before it
     int face_begin, face_end;
     int mblk_begin, mblk_end;       // blocks of the area / volume kernel (MESH_CHUNK faces each)
     int nlipid, pad1;               // lipids in the system (bulk-velocity removal)
@@ -141,7 +142,7 @@ __host__ __device__ __forceinline__ unsigned cell_code(const SysDev &s, int x, i
     return (tile << 6) | tile_spread2(unsigned(x) & 3u) | (tile_spread2(unsigned(y) & 3u) << 1) |
            (tile_spread2(unsigned(z) & 3u) << 2);
 }
-/* ids per system (tiles x 64); id cell_base + ncell_ids is the ghost id */
+/* ids per system (tiles x 64) */
 __host__ __device__ __forceinline__ unsigned ncell_ids(const SysDev &s) {
     return unsigned(s.ntile[0]) * unsigned(s.ntile[1]) * unsigned(s.ntile[2]) * 64u;
 }
@@ -162,7 +163,7 @@ struct __align__(16) Scalars {
     int nh_half;          // 1 between a Nose-Hoover first half and its second half
     unsigned int blk_counter, mesh_counter;
     unsigned int iters;   // completed steps or minimisation iterations (k_advance, k_reduce)
-    unsigned int pad3;
+    unsigned int scan_counter;
     long long step, rebuilds, since_rebuild, pad4;
 };
 
@@ -208,11 +209,17 @@ template<class R> struct KArgs {
     SysDev *sys;
     SysState *ss;
     int nsys, npad;
-    // radix sort scratch
+    // cell sort (see the rebuild chain): skey[0] = new cell id of each slot, skey[1] = slots by cell in arrival
+    // order, sval[0] = sorted slots, sval[1] = arrival rank in the cell; radix sort scratch of the cleanup
     uint32_t *skey[2];
     int *sval[2];
     int *counts, *digit_total, *inv;
-    int sort_passes, ntiles;
+    int ntiles;
+    int *ccnt;               // particles per cell, zero between rebuilds
+    int *tcnt, *tstart;      // per tile of 64 cells: particles (zero between rebuilds) and their prefix in its scan block
+    int *bsum;               // prefix of the scan blocks (SCAN_TILES tiles each)
+    int *gcnt;               // ghosts placed per system, zero between rebuilds
+    int nctile, nscan;       // tiles (padded to whole scan blocks), scan blocks
     // parameters
     double dt, kBT;
     R skin_half2;
@@ -223,7 +230,12 @@ template<class R> struct KArgs {
     int zero_bulk;           // remove the mean lipid velocity before integrating
     int nlist_lane;          // list-build form: 0 per cell of a warp, 1 per-lane 27-cell sweep, 2 two-phase
     const FFDev<R> *ff;      // force-field tables (global)
+    // conditional node whose value the step's last small kernel sets to the rebuild flag (graph capture; 0 = none)
+    cudaGraphConditionalHandle cond;
+    int has_cond;
 };
+
+constexpr int SCAN_TILES = 4096;  // cell tiles per block of the tile scan
 
 // host-side launchers (explicitly instantiated for float and double)
 template<class R> void launch_rebuild(const KArgs<R> &a, cudaStream_t st, bool gated);

@@ -490,7 +490,8 @@ template<class R> class Engine : public EngineBase {
             sd.Q = P.Q;
             off += npad_s;
             for (int dd = 0; dd < 3; ++dd) sd.ntile[dd] = (sd.nc[dd] + 3) / 4;
-            cbase += uint64_t(sd.ntile[0]) * uint64_t(sd.ntile[1]) * uint64_t(sd.ntile[2]) * 64u + 1;
+            cbase += uint64_t(sd.ntile[0]) * uint64_t(sd.ntile[1]) * uint64_t(sd.ntile[2]) * 64u;
+            sd.slot_shift = sd.off - int(b);
         }
         if (off >= MAX_SLOTS) return fail(ORBC_ERR_ARG, "upload: more than 2^27 particle slots");
         if (cbase >= (uint64_t(1) << 32) - 1) return fail(ORBC_ERR_ARG, "upload: more than 2^32 cells");
@@ -615,6 +616,11 @@ template<class R> class Engine : public EngineBase {
                 return fail(ORBC_ERR_NOMEM, "upload: device allocation failed");
         }
         ntiles = sort_tiles(npad);
+        nscan = int((total_cells / 64 + SCAN_TILES - 1) / SCAN_TILES);
+        const size_t nct = size_t(nscan) * SCAN_TILES;
+        if (ccnt.alloc(nct * 64) || tcnt.alloc(nct) || tstart.alloc(nct) || bsum.alloc(size_t(nscan)) ||
+            gcnt.alloc(size_t(nsys)))
+            return fail(ORBC_ERR_NOMEM, "upload: device allocation failed");
         if (epart.alloc(size_t(npad)) || faces.alloc(hfaces.size()) || ranges.alloc(size_t(total_cells)) ||
             soh.alloc(size_t(n)) || blk_sys.alloc(size_t(nb256)) || partial.alloc(size_t(npad / 32) * NPART) || gpartial.alloc(size_t(ngroups_total) * NPART) ||
             Sd.alloc(1) || sysd.alloc(size_t(nsys)) || ssd.alloc(size_t(nsys)) || counts.alloc(size_t(256) * ntiles) ||
@@ -645,6 +651,9 @@ template<class R> class Engine : public EngineBase {
         CK(cudaMemcpyAsync(blk_sys.p, hbs.data(), hbs.size() * sizeof(int), cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(sysd.p, hsys.data(), hsys.size() * sizeof(SysDev), cudaMemcpyHostToDevice, st));
         CK(cudaMemsetAsync(ranges.p, 0, size_t(total_cells) * sizeof(int2), st));
+        CK(cudaMemsetAsync(ccnt.p, 0, ccnt.n * sizeof(int), st));
+        CK(cudaMemsetAsync(tcnt.p, 0, tcnt.n * sizeof(int), st));
+        CK(cudaMemsetAsync(gcnt.p, 0, gcnt.n * sizeof(int), st));
         CK(cudaMemsetAsync(partial.p, 0, size_t(npad / 32) * NPART * sizeof(double), st));
         CK(cudaMemsetAsync(gpartial.p, 0, size_t(ngroups_total) * NPART * sizeof(double), st));
         CK(cudaMemsetAsync(epart.p, 0, size_t(npad) * sizeof(double), st));
@@ -660,10 +669,6 @@ template<class R> class Engine : public EngineBase {
         CK(cudaMemcpyAsync(ssd.p, hss.data(), hss.size() * sizeof(SysState), cudaMemcpyHostToDevice, st));
         build_ff();
         CK(cudaMemcpyAsync(ffd.p, &hff, sizeof(hff), cudaMemcpyHostToDevice, st));
-        // key bits -> radix passes
-        int bits = 1;
-        while (bits < 32 && (uint64_t(1) << bits) < total_cells) ++bits;
-        passes = (bits + 7) / 8;
         fill_args();
         CK(cudaStreamSynchronize(st));
         uploaded = true;
@@ -889,6 +894,7 @@ template<class R> class Engine : public EngineBase {
                 ntype.push_back(topo.type[size_t(h)]);
                 ntag.push_back(topo.tag[size_t(h)]);
             }
+            hsys[size_t(sy)].slot_shift = hsys[size_t(sy)].off - int(offs[size_t(sy)]);
             offs[size_t(sy) + 1] = k;
             hsys[size_t(sy)].nreal -= gone_here;
             hsys[size_t(sy)].nlipid -= gone_here;
@@ -1085,7 +1091,7 @@ template<class R> class Engine : public EngineBase {
         int k = (P.integrator == ORBC_INT_NOSE_HOOVER ? 4 : 2) + (has_mesh ? 1 : 0);
         return k + (graph_cond ? 1 : 0);
     }
-    int rebuild_launches() const { return 1 + 3 * passes + 1 + 1; }
+    int rebuild_launches() const { return 1 + 4 + 1 + 1; }
 
     /* Capture steps_per_graph steps into *exec (cond: the rebuild sits behind
      * a conditional node; otherwise the rebuild kernels are device-gated). */
@@ -1812,8 +1818,14 @@ template<class R> class Engine : public EngineBase {
         a.counts = counts.p;
         a.digit_total = dtot.p;
         a.inv = invd.p;
-        a.sort_passes = passes;
         a.ntiles = ntiles;
+        a.ccnt = ccnt.p;
+        a.tcnt = tcnt.p;
+        a.tstart = tstart.p;
+        a.bsum = bsum.p;
+        a.gcnt = gcnt.p;
+        a.nctile = nscan * SCAN_TILES;
+        a.nscan = nscan;
         a.dt = P.dt;
         a.kBT = P.kBT;
         a.skin_half2 = R(0.25 * P.skin * P.skin);
@@ -1891,7 +1903,7 @@ template<class R> class Engine : public EngineBase {
     bool graph_cond = false;
     int graph_steps = 0;
     bool uploaded = false, nh_primed = false, has_mesh = false, vcom_valid = false;
-    int nsys = 0, npad = 0, cap = 0, passes = 4, ntiles = 1, maxb = 0, maxf = 0, nfaces = 0, nmblk = 0;
+    int nsys = 0, npad = 0, cap = 0, ntiles = 1, nscan = 1, maxb = 0, maxf = 0, nfaces = 0, nmblk = 0;
     int64_t nhome = 0;
     uint64_t total_cells = 0;
     std::vector<SysDev> hsys;
@@ -1906,6 +1918,7 @@ template<class R> class Engine : public EngineBase {
     DevBuf<int4> faces;
     DevBuf<int2> ranges;
     DevBuf<int> soh, blk_sys, counts, dtot, invd, nnb, mesh_bs;
+    DevBuf<int> ccnt, tcnt, tstart, bsum, gcnt;  // cell sort
     DevBuf<double> mesh_part;
     DevBuf<uint32_t> nbr;
     DevBuf<Scalars> Sd;
