@@ -84,17 +84,12 @@ typedef struct {
     double bond_K[ORBC_MAX_BOND_TYPES];
     double bond_r0[ORBC_MAX_BOND_TYPES];
     double bond_R[ORBC_MAX_BOND_TYPES];
-    /* kernel forms 0..127 (bits 3 and 4 not both set).  Bits 3-4 = how
-       the neighbour list is built: 0 per cell of a warp, 32 candidates at a
-       time, entries placed by prefix count; 1
-       per-particle 27-cell sweeps; 2 per warp in two phases (accept masks per
-       particle, then every lane writes its own column) -- all three write the
-       same list.  Bit 6 (64) = compensated (Kahan)
-       summation of each particle's force and torque, also in the forces
-       hook.  Bits 0, 1, 2 and 5 chose between forms of the force loop; one
-       loop, whose row batches follow the number of particles, now serves them
-       all: they are accepted and change nothing.  orbc_gpu_autotune picks the
-       forms per workload */
+    /* kernel forms 0..127 (bits 3 and 4 not both set).  Bit 6 (64) =
+       compensated (Kahan) summation of each particle's force and torque, also
+       in the forces hook.  The other bits chose between forms of the force
+       loop (0, 1, 2, 5) and of the neighbour-list build (3, 4) with the same
+       results; one force loop and one list build, which follow the number of
+       particles, now serve them all: they are accepted and change nothing */
     int kernel_variant;
     /* 1: remove each system's mean lipid velocity between the force
        evaluation and the integrator every step, as the disabled call

@@ -18,6 +18,7 @@
 #include "orbc_device.cuh"
 
 #include <cstdio>
+#include <type_traits>
 
 namespace orbc {
 
@@ -449,255 +450,38 @@ template<class R> __device__ __forceinline__ void nlist_finalise(const KArgs<R> 
     }
 }
 
-template<class R> __global__ void __launch_bounds__(128) k_nlist(KArgs<R> a, int gated) {
-    using T4 = typename Vec<R>::T4;
-    if (gated && !__ldcg(&a.S->rebuild)) return;
-    constexpr int CAND = sizeof(T4) == 16 ? 384 : 192;  // staged candidates per warp and pass
-    constexpr int NLW = 4;                                // warps per block
-    __shared__ float rl2s[256], ri2s[256];
-    __shared__ T4 s_pos[NLW][CAND];
-    __shared__ int s_j[NLW][CAND];
-    __shared__ unsigned char s_code[NLW][CAND];           // shift code of the candidate's cell (0..26)
-    __shared__ int s_off[NLW][28], s_beg[NLW][27];
-    const int warp = threadIdx.x >> 5;
-    for (int k = threadIdx.x; k < 256; k += blockDim.x) {
-        rl2s[k] = __ldg(&a.ff->rlist2[k]);
-        ri2s[k] = __ldg(&a.ff->rin2[k]);
-    }
-    __syncthreads();
-    const int cur = 1 - __ldcg(&a.S->cur), lp = 1 - __ldcg(&a.S->lp);
-    const int n = a.npad;
-    int maxc = 0;
-    // n is a multiple of the block size, so whole warps stay in the loop together
-    const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const T4 p = a.pos[cur][i];
-        const int ty = w_type(wbits(p.w));
-        const bool real = ty != GHOST;
-        const SysDev &sd = a.sys[a.blk_sys[i / SYS_PAD]];  // one system per warp (SYS_PAD-aligned)
-        const int c = a.cell[lp][i];
-        const int cc[3] = {cx_of(c), cy_of(c), cz_of(c)};
-        const R L[3] = {lc_of<R>(sd, 0), lc_of<R>(sd, 1), lc_of<R>(sd, 2)};
-        // Entries inside the pair's interaction range fill rows 0, 1, ... of
-        // this slot's column; skin-shell entries fill rows cap-1, cap-2, ...
-        int nin = 0, nout = 0, total = 0;
-        // Candidate j seen from i's cell: o_j + d * Lc (d = cell_j - cell_i);
-        // x_i - x_j = o_i - (o_j + d * Lc).  Both list-build forms use these
-        // two functions, so they accept the same pairs.
-        auto shifted = [&](const T4 &q, int dx, int dy, int dz) {
-            T4 r = q;
-            r.x = q.x + R(dx) * L[0];
-            r.y = q.y + R(dy) * L[1];
-            r.z = q.z + R(dz) * L[2];
-            return r;
-        };
-        auto dist2 = [&](const T4 &pi, const T4 &qs) {
-            const R ex = pi.x - qs.x, ey = pi.y - qs.y, ez = pi.z - qs.z;
-            return ex * ex + ey * ey + ez * ez;
-        };
-        auto test = [&](int j, const T4 &q, int dx, int dy, int dz) {
-            const int tj = w_type(wbits(q.w));
-            const float rl2 = rl2s[ty * 16 + tj];
-            if (!(rl2 > 0.f)) return;
-            const R r2 = dist2(p, shifted(q, dx, dy, dz));
-            if (r2 < R(rl2)) {
-                const uint32_t ent = uint32_t(j) | (uint32_t((dx + 1) + 3 * (dy + 1) + 9 * (dz + 1)) << NB_SHIFT);
-                if (nin + nout < a.cap) {
-                    if (r2 < R(ri2s[ty * 16 + tj]))
-                        a.nbr[nbr_index(i, nin++, a.cap)] = ent;
-                    else
-                        a.nbr[nbr_index(i, a.cap - 1 - nout++, a.cap)] = ent;
-                }
-                ++total;
-            }
-        };
-        // Form 0 (warp sweep): consecutive slots sit in a few neighbouring
-        // cells (cell ids follow tiles).  For each distinct cell of the warp,
-        // 27 lanes fetch the ranges of its 27 neighbour cells, a warp scan
-        // turns them into offsets and the candidates are staged in shared
-        // memory (CAND per pass, all loads issued together); then for each
-        // particle in that cell the 32 lanes test 32 candidates at a time and
-        // accepted entries are placed by ballot and prefix count.  Form 1
-        // (per-lane sweep): every lane walks its own 27 cells.
-        bool swept = false;
-        if (!a.nlist_lane) {
-            swept = true;
-            const int kme = cc[0] | (cc[1] << 11) | (cc[2] << 22);
-            int *off = s_off[warp];
-            int *beg = s_beg[warp];
-            unsigned todo = __ballot_sync(0xffffffffu, real);
-            while (todo) {
-                // the lanes in one cell share its candidates
-                const int kd = __shfl_sync(0xffffffffu, kme, __ffs(todo) - 1);
-                const unsigned grp = __ballot_sync(0xffffffffu, real && kme == kd);
-                todo &= ~grp;
-                const int xd = kd & 2047, yd = (kd >> 11) & 2047, zd = (kd >> 22) & 1023;
-                int2 rg = make_int2(0, 0);
-                if (lane < 27) {
-                    int x = xd + lane % 3 - 1, y = yd + (lane / 3) % 3 - 1, z = zd + lane / 9 - 1;
-                    bool ok = true;
-                    if (sd.per[0]) x = x < 0 ? x + sd.nc[0] : (x >= sd.nc[0] ? x - sd.nc[0] : x);
-                    else ok = ok && x >= 0 && x < sd.nc[0];
-                    if (sd.per[1]) y = y < 0 ? y + sd.nc[1] : (y >= sd.nc[1] ? y - sd.nc[1] : y);
-                    else ok = ok && y >= 0 && y < sd.nc[1];
-                    if (sd.per[2]) z = z < 0 ? z + sd.nc[2] : (z >= sd.nc[2] ? z - sd.nc[2] : z);
-                    else ok = ok && z >= 0 && z < sd.nc[2];
-                    if (ok) rg = a.ranges[sd.cell_base + cell_code(sd, x, y, z)];
-                }
-                const int cnt = rg.y > rg.x ? rg.y - rg.x : 0;
-                int inc = cnt;  // inclusive warp scan
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += t;
-                }
-                if (lane < 27) {
-                    off[lane] = inc - cnt;
-                    beg[lane] = rg.x;
-                }
-                const int total_c = __shfl_sync(0xffffffffu, inc, 31);
-                if (lane == 0) off[27] = total_c;
-                __syncwarp();
-                // per-particle counters of this cell's particles, carried across passes
-                int cin = 0, cout = 0, ctot = 0;
-                for (int c0 = 0; c0 < total_c; c0 += CAND) {
-                    const int nch = min(CAND, total_c - c0);
-                    for (int t = lane; t < nch; t += 32) {
-                        const int idx = c0 + t;
-                        int l = 0;  // last neighbour cell with off[l] <= idx
-#pragma unroll
-                        for (int step = 16; step > 0; step >>= 1)
-                            if (l + step < 27 && off[l + step] <= idx) l += step;
-                        const int j = beg[l] + (idx - off[l]);
-                        s_pos[warp][t] = shifted(a.pos[cur][j], l % 3 - 1, (l / 3) % 3 - 1, l / 9 - 1);
-                        s_j[warp][t] = j;
-                        s_code[warp][t] = (unsigned char)l;
-                    }
-                    __syncwarp();
-                    for (unsigned g = grp; g; g &= g - 1u) {
-                        const int il = __ffs(g) - 1;
-                        T4 pi = p;
-                        pi.x = __shfl_sync(0xffffffffu, p.x, il);
-                        pi.y = __shfl_sync(0xffffffffu, p.y, il);
-                        pi.z = __shfl_sync(0xffffffffu, p.z, il);
-                        const int ti = __shfl_sync(0xffffffffu, ty, il);
-                        const int gi = i - lane + il;
-                        int qin = __shfl_sync(0xffffffffu, cin, il), qout = __shfl_sync(0xffffffffu, cout, il);
-                        int qtot = __shfl_sync(0xffffffffu, ctot, il);
-                        uint32_t *col = a.nbr + nbr_index(gi, 0, a.cap);  // row k of gi at col[32 k]
-                        // lipid-lipid pairs (the bulk) take their cutoffs from registers
-                        const float rl2_ll = rl2s[ti * 16], ri2_ll = ri2s[ti * 16];
-                        for (int b0 = 0; b0 < nch; b0 += 32) {
-                            const int t = b0 + lane;
-                            bool acc = false, inner = false;
-                            uint32_t ent = 0;
-                            if (t < nch) {
-                                const int j = s_j[warp][t];
-                                const T4 q = s_pos[warp][t];
-                                const int tj = w_type(wbits(q.w));
-                                const float rl2 = tj == 0 ? rl2_ll : rl2s[ti * 16 + tj];
-                                if (j != gi && rl2 > 0.f) {
-                                    const R r2 = dist2(pi, q);
-                                    if (r2 < R(rl2)) {
-                                        acc = true;
-                                        inner = r2 < R(tj == 0 ? ri2_ll : ri2s[ti * 16 + tj]);
-                                        ent = uint32_t(j) | (uint32_t(s_code[warp][t]) << NB_SHIFT);
-                                    }
-                                }
-                            }
-                            const unsigned ma = __ballot_sync(0xffffffffu, acc);
-                            const unsigned mi = __ballot_sync(0xffffffffu, acc && inner);
-                            // entries past the capacity are counted, not written
-                            unsigned mw = ma;
-                            if (qin + qout + __popc(ma) > a.cap)
-                                mw = __ballot_sync(0xffffffffu, acc && qin + qout + __popc(ma & lt) < a.cap);
-                            if ((mw >> lane) & 1u) {
-                                const int row = inner ? qin + __popc(mi & mw & lt)
-                                                      : a.cap - 1 - (qout + __popc(~mi & mw & lt));
-                                col[32 * row] = ent;
-                            }
-                            const int win = __popc(mi & mw);
-                            qin += win;
-                            qout += __popc(mw) - win;
-                            qtot += __popc(ma);
-                        }
-                        if (lane == il) {
-                            cin = qin;
-                            cout = qout;
-                            ctot = qtot;
-                        }
-                    }
-                    __syncwarp();
-                }
-                if (grp & (1u << lane)) {
-                    nin = cin;
-                    nout = cout;
-                    total = ctot;
-                }
-            }
-        }
-        if (!swept && real) {
-            for (int dz = -1; dz <= 1; ++dz) {
-                int z = cc[2] + dz;
-                if (sd.per[2]) {
-                    z = z < 0 ? z + sd.nc[2] : (z >= sd.nc[2] ? z - sd.nc[2] : z);
-                } else if (z < 0 || z >= sd.nc[2]) {
-                    continue;
-                }
-                for (int dy = -1; dy <= 1; ++dy) {
-                    int y = cc[1] + dy;
-                    if (sd.per[1]) {
-                        y = y < 0 ? y + sd.nc[1] : (y >= sd.nc[1] ? y - sd.nc[1] : y);
-                    } else if (y < 0 || y >= sd.nc[1]) {
-                        continue;
-                    }
-                    for (int dx = -1; dx <= 1; ++dx) {
-                        int x = cc[0] + dx;
-                        if (sd.per[0]) {
-                            x = x < 0 ? x + sd.nc[0] : (x >= sd.nc[0] ? x - sd.nc[0] : x);
-                        } else if (x < 0 || x >= sd.nc[0]) {
-                            continue;
-                        }
-                        const int2 rg = a.ranges[sd.cell_base + cell_code(sd, x, y, z)];
-                        for (int j = rg.x; j < rg.y; ++j)
-                            if (j != i) test(j, a.pos[cur][j], dx, dy, dz);
-                    }
-                }
-            }
-        }
-        a.nnb[i] = real ? (nin | (nout << 16)) : 0;
-        maxc = max(maxc, total);
-    }
-    nlist_finalise(a, maxc, cur, lp);
-}
-
-/* Form 2 of the list build (two phases per warp).  The distinct cells of a
- * warp's particles are fetched as in form 0 -- 27 lanes fetch a cell's
- * neighbour ranges -- and each cell's candidates are staged pre-shifted into
- * that cell's frame, padded with ghosts (never accepted) to a multiple of
- * 32.  Phase 1: for two particles of the cell at a time the warp tests 32
- * candidates per ballot pair, branch-free (one staged load serves both
- * particles), and each particle's own lane keeps the accept masks (in range
- * at all / inside the interaction range) in registers.  The candidates' list
- * entries stay staged in shared memory for as many cells as fit, so that
- * phase 2 -- every lane expands its masks in candidate order into its own
- * column -- runs for most warps once, with all their lanes.  The candidates,
- * their order and the arithmetic are those of forms 0 and 1, so all three
- * forms write the same rows. */
-template<class R> __device__ __forceinline__ R ghost_w_of();  // the w word of a ghost's position
-template<> __device__ __forceinline__ float ghost_w_of<float>() { return __int_as_float(GHOST); }
-template<> __device__ __forceinline__ double ghost_w_of<double>() { return __longlong_as_double((long long)GHOST); }
+/* Neighbour list, in two phases per warp.  For each distinct cell of a
+ * warp's particles 27 lanes fetch the neighbour cells' ranges and the
+ * candidates are staged pre-shifted into that cell's frame, padded (never
+ * accepted) to a multiple of 32.  Phase 1: for two particles of the cell at a
+ * time the warp tests 32 candidates per ballot pair, branch-free (one staged
+ * load serves both particles), and each particle's own lane keeps the accept
+ * masks (in range at all / inside the interaction range) in registers; where
+ * particles and candidates are of types 0..3, which share one list cutoff, the
+ * cutoffs are two registers instead of two table lookups per test.  The
+ * candidates' list entries stay staged in shared memory for as many cells as
+ * fit, so that phase 2 -- every lane expands its masks in candidate order into
+ * its own column, inner rows upwards and shell rows downwards -- runs for most
+ * warps once, with all their lanes.
+ *
+ * SW warps share 32 slots, each taking 32 / SW of their particles: one warp's
+ * chain of cells, ballots and expansions is some 80 thousand cycles long, which
+ * is the time of the build while the GPU is not full. */
+// Bound by instruction issue (70 % of peak, 9.0 thousand warp instructions per
+// 32 slots, half of them cell ranges and staging).  1.0M-particle cell 0.357 ->
+// 0.348 ms, 1.0M lipids in 23 vesicles 0.359 -> 0.332 ms against table lookups
+// and a single expansion loop; a third copy of phase 1 for lipids alone made
+// the cell with anchors slower (0.379 ms: the instruction cache).
 // 7 resident blocks per SM: the staging below (about 31 KB per block in FP32)
 // and at most 72 registers; more warps in flight beat fewer passes per warp
-template<class R> __global__ void __launch_bounds__(128, 7) k_nlist2(KArgs<R> a, int gated) {
+template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArgs<R> a, int gated) {
     using T4 = typename Vec<R>::T4;
     if (gated && !__ldcg(&a.S->rebuild)) return;
     constexpr int NLW = 4;                                // warps per block
     constexpr int MB = 8;                                 // accept masks (32 candidates each) per lane
     constexpr int REG = 32 * MB;                          // candidates of one cell (or chunk) per phase 1
     constexpr int SE = sizeof(T4) == 16 ? 768 : 512;      // list entries staged per warp until phase 2
-    __shared__ float2 s_cut[256];                         // (list cutoff^2, range cutoff^2) per type pair
+    __shared__ float2 s_cut[256];                         // (list cutoff^2, inner cutoff^2) per type pair
     __shared__ T4 s_pos[NLW][REG];                        // the current cell's candidates
     __shared__ uint32_t s_ent[NLW][SE];                   // j | shift code of its cell << NB_SHIFT
     __shared__ int s_off[NLW][28], s_beg[NLW][27];
@@ -706,16 +490,19 @@ template<class R> __global__ void __launch_bounds__(128, 7) k_nlist2(KArgs<R> a,
         s_cut[k] = make_float2(__ldg(&a.ff->rlist2[k]), __ldg(&a.ff->rin2[k]));
     __syncthreads();
     const int cur = 1 - __ldcg(&a.S->cur), lp = 1 - __ldcg(&a.S->lp);
-    // the grid covers npad (a multiple of the block size) once
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    // the grid covers npad (a multiple of the block size) SW times
+    const int wid = blockIdx.x * NLW + warp;
+    const int i = wid / SW * 32 + lane;
+    const bool mine = SW == 1 || lane / (32 / SW) == wid % SW;
     const T4 p = a.pos[cur][i];
     const int ty = w_type(wbits(p.w));
-    const bool real = ty != GHOST;
+    const bool real = ty != GHOST && mine;
     const SysDev &sd = a.sys[a.blk_sys[i / SYS_PAD]];  // one system per warp (SYS_PAD-aligned)
     const int c = a.cell[lp][i];
     const int cc[3] = {cx_of(c), cy_of(c), cz_of(c)};
     const R L[3] = {lc_of<R>(sd, 0), lc_of<R>(sd, 1), lc_of<R>(sd, 2)};
-    // the expressions of k_nlist's shifted() and dist2()
+    // Candidate j seen from i's cell: o_j + d * Lc (d = cell_j - cell_i);
+    // x_i - x_j = o_i - (o_j + d * Lc).
     auto shifted = [&](const T4 &q, int dx, int dy, int dz) {
         T4 r = q;
         r.x = q.x + R(dx) * L[0];
@@ -733,8 +520,8 @@ template<class R> __global__ void __launch_bounds__(128, 7) k_nlist2(KArgs<R> a,
     T4 *sp = s_pos[warp];
     uint32_t *se = s_ent[warp];
     uint32_t *col = a.nbr + nbr_index(i, 0, a.cap);  // row k of slot i at col[32 k]
-    const R ghost_w = ghost_w_of<R>();
     const int cap = a.cap;
+    const float2 cut_ll = s_cut[0];
     int qin = 0, qout = 0, qtot = 0;
     // neighbour ranges of cell kd -> off/beg; returns the candidate count
     auto fetch = [&](int kd) {
@@ -766,8 +553,9 @@ template<class R> __global__ void __launch_bounds__(128, 7) k_nlist2(KArgs<R> a,
         __syncwarp();
         return __shfl_sync(0xffffffffu, inc, 31);
     };
-    // candidates [c0, c0 + nch) of the fetched cell -> sp[0 ...] and se[ebase ...]
+    // candidates [c0, c0 + nch) of the fetched cell -> sp[0 ...] and se[ebase ...]; the or of their types
     auto stage = [&](int c0, int nch, int ebase) {
+        unsigned types = 0;
 #pragma unroll 4
         for (int t = lane; t < nch; t += 32) {
             const int idx = c0 + t;
@@ -776,25 +564,29 @@ template<class R> __global__ void __launch_bounds__(128, 7) k_nlist2(KArgs<R> a,
             for (int step = 16; step > 0; step >>= 1)
                 if (l + step < 27 && off[l + step] <= idx) l += step;
             const int j = beg[l] + (idx - off[l]);
-            sp[t] = shifted(a.pos[cur][j], l % 3 - 1, (l / 3) % 3 - 1, l / 9 - 1);
+            const T4 q = a.pos[cur][j];
+            types |= w_type(wbits(q.w));
+            sp[t] = shifted(q, l % 3 - 1, (l / 3) % 3 - 1, l / 9 - 1);
             se[ebase + t] = uint32_t(j) | (uint32_t(l) << NB_SHIFT);
         }
-        if (nch + lane < ((nch + 31) & ~31)) {  // ghosts up to a multiple of 32: never accepted
+        if (nch + lane < ((nch + 31) & ~31)) {  // far away: never accepted
             T4 z;
-            z.x = z.y = z.z = R(0);
-            z.w = ghost_w;
+            z.x = z.y = z.z = R(1e18);
+            z.w = R(0);
             sp[nch + lane] = z;
         }
         __syncwarp();
+        return __reduce_or_sync(0xffffffffu, types);
     };
     uint32_t macc[MB], minn[MB];
-    // phase 1 for the particles grp, two per pass, over the staged candidates [0, nch), nch <= REG;
-    // ts: the owning lane's own staged index (self is not a neighbour), -1 if absent
-    auto phase1 = [&](unsigned grp, int nch, int ts) {
+    // phase 1 for the particles grp, two per pass, over the staged candidates [0, nch), nch <= REG.
+    // ONE: one list and one inner cutoff; otherwise cutoffs by type pair
+    auto phase1 = [&](unsigned grp, int nch, auto one_cutoff) {
+        constexpr bool ONE = decltype(one_cutoff)::value;
         for (unsigned g = grp; g;) {
-            const int il = __ffs(g) - 1;
+            const int il = __ffs(int(g)) - 1;
             g &= g - 1u;
-            const int il2 = g ? __ffs(g) - 1 : il;  // the second particle of the pass (il again if none)
+            const int il2 = g ? __ffs(int(g)) - 1 : il;  // the second particle of the pass (il again if none)
             if (g) g &= g - 1u;
             T4 pi = p, pi2 = p;
             pi.x = __shfl_sync(0xffffffffu, p.x, il);
@@ -803,26 +595,22 @@ template<class R> __global__ void __launch_bounds__(128, 7) k_nlist2(KArgs<R> a,
             pi2.x = __shfl_sync(0xffffffffu, p.x, il2);
             pi2.y = __shfl_sync(0xffffffffu, p.y, il2);
             pi2.z = __shfl_sync(0xffffffffu, p.z, il2);
-            const int ti = __shfl_sync(0xffffffffu, ty, il) * 16;
-            const int tsi = __shfl_sync(0xffffffffu, ts, il);
-            const int ti2 = __shfl_sync(0xffffffffu, ty, il2) * 16;
-            const int tsi2 = __shfl_sync(0xffffffffu, ts, il2);
+            const int ti = ONE ? 0 : __shfl_sync(0xffffffffu, ty, il) * 16;
+            const int ti2 = ONE ? 0 : __shfl_sync(0xffffffffu, ty, il2) * 16;
 #pragma unroll
             for (int b = 0; b < MB; ++b) {
                 if (b * 32 < nch) {
-                    const int t = b * 32 + lane;
-                    const T4 q = sp[t];
-                    const int tj = w_type(wbits(q.w));
-                    const float2 cut = s_cut[ti + tj];
-                    const float2 cut2 = s_cut[ti2 + tj];
+                    const T4 q = sp[b * 32 + lane];
+                    const int tj = ONE ? 0 : w_type(wbits(q.w));
+                    const float2 cut = ONE ? cut_ll : s_cut[ti + tj];
+                    const float2 cut2 = ONE ? cut_ll : s_cut[ti2 + tj];
                     const R r2 = dist2(pi, q);
                     const R r2b = dist2(pi2, q);
-                    const bool acc = t != tsi && r2 < R(cut.x);
-                    const bool acc2 = t != tsi2 && r2b < R(cut2.x);
-                    const unsigned ma = __ballot_sync(0xffffffffu, acc);
-                    const unsigned mi = __ballot_sync(0xffffffffu, acc && r2 < R(cut.y));
-                    const unsigned ma2 = __ballot_sync(0xffffffffu, acc2);
-                    const unsigned mi2 = __ballot_sync(0xffffffffu, acc2 && r2b < R(cut2.y));
+                    // inner cutoff <= list cutoff; a particle's own bit is cleared in phase 2
+                    const unsigned ma = __ballot_sync(0xffffffffu, r2 < R(cut.x));
+                    unsigned mi = __ballot_sync(0xffffffffu, r2 < R(cut.y));
+                    const unsigned ma2 = __ballot_sync(0xffffffffu, r2b < R(cut2.x));
+                    unsigned mi2 = __ballot_sync(0xffffffffu, r2b < R(cut2.y));
                     if (lane == il) {
                         macc[b] = ma;
                         minn[b] = mi;
@@ -835,28 +623,74 @@ template<class R> __global__ void __launch_bounds__(128, 7) k_nlist2(KArgs<R> a,
             }
         }
     };
-    int mybase = 0;  // where this lane's candidates start in se
+    int mybase = 0;   // where this lane's candidates start in se
+    int myself = -1;  // this lane's own candidate index, -1 if absent
     // phase 2: this lane's accepted candidates, in order; the masks are cleared
     auto phase2 = [&]() {
+        int nall = 0, ninn = 0;
 #pragma unroll
         for (int b = 0; b < MB; ++b) {
-            unsigned m = macc[b];
-            const unsigned mi = minn[b];
-            while (m) {
-                const int bit = __ffs(m) - 1;
-                m &= m - 1u;
-                const uint32_t e = se[mybase + b * 32 + bit];
-                const bool in = (mi >> bit) & 1u;
-                if (qin + qout < cap) {
-                    col[32 * (in ? qin : cap - 1 - qout)] = e;
-                    qin += in;
-                    qout += !in;
-                }
-                ++qtot;
-            }
-            macc[b] = minn[b] = 0u;
+            const unsigned own = (myself >> 5) == b ? 1u << (myself & 31) : 0u;
+            macc[b] &= ~own;
+            minn[b] &= ~own;
+            nall += __popc(macc[b]);
+            ninn += __popc(minn[b]);
         }
+        qtot += nall;
+        if (!__any_sync(0xffffffffu, qin + qout + nall > cap)) {
+            uint32_t *up = col + 32 * qin;
+            uint32_t *down = col + 32 * (cap - 1 - qout);
+            qin += ninn;
+            qout += nall - ninn;
+#pragma unroll
+            for (int b = 0; b < MB; ++b) {
+                for (unsigned m = minn[b]; m; m &= m - 1u) {
+                    *up = se[mybase + b * 32 + __ffs(int(m)) - 1];
+                    up += 32;
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < MB; ++b) {
+                for (unsigned m = macc[b] & ~minn[b]; m; m &= m - 1u) {
+                    *down = se[mybase + b * 32 + __ffs(int(m)) - 1];
+                    down -= 32;
+                }
+            }
+        } else {  // entries past the capacity are counted, not written
+#pragma unroll
+            for (int b = 0; b < MB; ++b) {
+                for (unsigned m = macc[b]; m; m &= m - 1u) {
+                    const int bit = __ffs(int(m)) - 1;
+                    const bool in = (minn[b] >> bit) & 1u;
+                    if (qin + qout < cap) {
+                        col[32 * (in ? qin : cap - 1 - qout)] = se[mybase + b * 32 + bit];
+                        qin += in;
+                        qout += !in;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < MB; ++b) macc[b] = minn[b] = 0u;
+        myself = -1;
         __syncwarp();  // every lane is done with se before it is restaged
+    };
+    auto test = [&](unsigned grp, int nch, unsigned types) {
+        types |= __reduce_or_sync(0xffffffffu, (grp >> lane) & 1u ? unsigned(ty) : 0u);
+        if (types < 4u && a.uniform_cut) {
+            phase1(grp, nch, std::true_type());
+            if (types) {  // the inner partners of types 0..3 are the lipids
+#pragma unroll
+                for (int b = 0; b < MB; ++b) {
+                    if (b * 32 < nch) {
+                        const unsigned m = __ballot_sync(0xffffffffu, w_type(wbits(sp[b * 32 + lane].w)) == 0);
+                        if ((grp >> lane) & 1u) minn[b] &= m;
+                    }
+                }
+            }
+        } else {
+            phase1(grp, nch, std::false_type());
+        }
     };
 #pragma unroll
     for (int b = 0; b < MB; ++b) macc[b] = minn[b] = 0u;
@@ -864,11 +698,12 @@ template<class R> __global__ void __launch_bounds__(128, 7) k_nlist2(KArgs<R> a,
     unsigned pend = 0u;  // lanes whose masks refer to se
     int eused = 0;       // entries staged in se
     while (todo) {
-        const int kd = __shfl_sync(0xffffffffu, kme, __ffs(todo) - 1);
+        const int kd = __shfl_sync(0xffffffffu, kme, __ffs(int(todo)) - 1);
         const unsigned grp = __ballot_sync(0xffffffffu, real && kme == kd) & todo;
         const int total_c = fetch(kd);
         todo &= ~grp;
         const int ts = off[13] + (i - beg[13]);
+        const bool member = (grp >> lane) & 1u;
         if (total_c > REG) {  // in chunks of REG, each placed at once
             if (pend) phase2();
             pend = 0u;
@@ -876,8 +711,8 @@ template<class R> __global__ void __launch_bounds__(128, 7) k_nlist2(KArgs<R> a,
             mybase = 0;
             for (int c0 = 0; c0 < total_c; c0 += REG) {
                 const int nch = min(REG, total_c - c0);
-                stage(c0, nch, 0);
-                phase1(grp, nch, (ts >= c0 && ts < c0 + nch) ? ts - c0 : -1);
+                test(grp, nch, stage(c0, nch, 0));
+                if (member) myself = (ts >= c0 && ts < c0 + nch) ? ts - c0 : -1;
                 phase2();
             }
             continue;
@@ -887,15 +722,30 @@ template<class R> __global__ void __launch_bounds__(128, 7) k_nlist2(KArgs<R> a,
             pend = 0u;
             eused = 0;
         }
-        stage(0, total_c, eused);
-        phase1(grp, total_c, ts);
-        if ((grp >> lane) & 1u) mybase = eused;
+        test(grp, total_c, stage(0, total_c, eused));
+        if (member) {
+            mybase = eused;
+            myself = ts;
+        }
         eused += total_c;
         pend |= grp;
     }
     if (pend) phase2();
-    a.nnb[i] = real ? (qin | (qout << 16)) : 0;
+    if (mine) a.nnb[i] = real ? (qin | (qout << 16)) : 0;
     nlist_finalise(a, real ? qtot : 0, cur, lp);
+}
+
+/* As many warps per 32 slots (4, 2 or 1) as are all resident at once (28 per
+ * SM, 152 SMs): there the chain of one warp sets the time.  Four / two / one warps:
+ * 2,048 particles 17 / 20 / 25 us, 32,768: 27 / 31 / 41 us, 131,946 (one fits): 86 / 66 / 59 us. */
+template<class R> void launch_nlist(const KArgs<R> &a, cudaStream_t st, int gated) {
+    const int nw = a.npad / 32, room = 152 * 28;  // nw is a multiple of 8
+    if (nw * 4 <= room)
+        k_nlist<R, 4><<<nw, 128, 0, st>>>(a, gated);
+    else if (nw * 2 <= room)
+        k_nlist<R, 2><<<nw / 2, 128, 0, st>>>(a, gated);
+    else
+        k_nlist<R, 1><<<nw / 4, 128, 0, st>>>(a, gated);
 }
 
 static int grid_for(int64_t n, int per_block = 256) {
@@ -921,10 +771,7 @@ template<class R> void launch_rebuild_stage(const KArgs<R> &a, cudaStream_t st, 
             k_gather<R><<<g, 256, 0, st>>>(a, gated ? 1 : 0);
             break;
         default:
-            if (a.nlist_lane == 2)
-                k_nlist2<R><<<(a.npad + 127) / 128, 128, 0, st>>>(a, gated ? 1 : 0);
-            else
-                k_nlist<R><<<(a.npad + 127) / 128, 128, 0, st>>>(a, gated ? 1 : 0);
+            launch_nlist<R>(a, st, gated ? 1 : 0);
             break;
     }
 }

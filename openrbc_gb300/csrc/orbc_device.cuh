@@ -228,7 +228,7 @@ template<class R> struct KArgs {
     int kahan;               // compensated sums of each particle's force and torque
     int carry_forces;        // forces / torques persist between kernels (Nose-Hoover)
     int zero_bulk;           // remove the mean lipid velocity before integrating
-    int nlist_lane;          // list-build form: 0 per cell of a warp, 1 per-lane 27-cell sweep, 2 two-phase
+    int uniform_cut;         // one list cutoff for all pairs of types 0..3, one inner cutoff for those with a lipid
     const FFDev<R> *ff;      // force-field tables (global)
     // conditional node whose value the step's last small kernel sets to the rebuild flag (graph capture; 0 = none)
     cudaGraphConditionalHandle cond;

@@ -1832,7 +1832,11 @@ template<class R> class Engine : public EngineBase {
         a.seed = P.seed;
         a.rebuild_every = P.rebuild_every;
         a.kahan = (P.kernel_variant & 64) ? 1 : 0;
-        a.nlist_lane = (P.kernel_variant >> 3) & 3;
+        a.uniform_cut = 1;
+        for (int ti = 0; ti < 4; ++ti)
+            for (int tj = 0; tj < 4; ++tj)
+                if (hff.rlist2[ti * 16 + tj] != hff.rlist2[0] || hff.rin2[ti * 16 + tj] != (tj == 0 ? hff.rin2[0] : 0.f))
+                    a.uniform_cut = 0;
         a.carry_forces = P.integrator == ORBC_INT_NOSE_HOOVER ? 1 : 0;
         a.zero_bulk = P.zero_bulk ? 1 : 0;
         a.ff = ffd.p;
