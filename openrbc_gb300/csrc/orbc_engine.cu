@@ -1086,10 +1086,9 @@ template<class R> class Engine : public EngineBase {
     /* Langevin without energy or bulk-velocity removal: no per-step sums */
     bool lite() const { return P.integrator == ORBC_INT_LANGEVIN && !P.energy && !P.zero_bulk; }
     /* per step: the force kernel and k_advance (lite) or k_reduce; Nose-Hoover
-     * adds k_nh_initial and its k_reduce; the mesh kernel; the condition kernel */
+     * adds k_nh_initial and its k_reduce; the mesh kernel */
     int fixed_launches_per_step() const {
-        int k = (P.integrator == ORBC_INT_NOSE_HOOVER ? 4 : 2) + (has_mesh ? 1 : 0);
-        return k + (graph_cond ? 1 : 0);
+        return (P.integrator == ORBC_INT_NOSE_HOOVER ? 4 : 2) + (has_mesh ? 1 : 0);
     }
     int rebuild_launches() const { return 1 + 4 + 1 + 1; }
 
@@ -1098,20 +1097,28 @@ template<class R> class Engine : public EngineBase {
     int capture_graph(int steps_per_graph, cudaGraphExec_t *exec, bool *cond) {
         cudaGraphExec_t gexec = nullptr;
         cudaGraph_t g = nullptr;
-        // conditional rebuild: [pre] -> set_cond -> IF{rebuild} -> [mesh] -> step kernel
+        // conditional rebuild: IF{rebuild} -> [mesh] -> step kernel; the condition is set by the last small kernel
+        // of the step before (k_advance, k_reduce; Nose-Hoover: k_reduce of the step's own first half), and by a
+        // kernel of its own for the first Langevin step
         bool ok = cudaGraphCreate(&g, 0) == cudaSuccess;
         std::vector<cudaGraph_t> bodies;
         if (ok) {
             ok = cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) ==
                  cudaSuccess;
+            std::vector<cudaGraphConditionalHandle> hc(static_cast<size_t>(steps_per_graph));
+            for (cudaGraphConditionalHandle &h : hc)
+                ok = ok && cudaGraphConditionalHandleCreate(&h, g, 0, 0) == cudaSuccess;
+            const bool nh = P.integrator == ORBC_INT_NOSE_HOOVER;
+            KArgs<R> ak = a;
             for (int k = 0; ok && k < steps_per_graph; ++k) {
-                cudaGraphConditionalHandle hc;
-                if (cudaGraphConditionalHandleCreate(&hc, g, 0, 0) != cudaSuccess) {
-                    ok = false;
-                    break;
+                if (nh) {
+                    ak.cond = hc[size_t(k)];
+                    ak.has_cond = 1;
+                    launch_nh_initial<R>(ak, st);
+                    ak.has_cond = 0;
+                } else if (k == 0) {
+                    launch_set_cond(hc[0], a.S, st);
                 }
-                if (P.integrator == ORBC_INT_NOSE_HOOVER) launch_nh_initial<R>(a, st);
-                launch_set_cond(hc, a.S, st);
                 cudaStreamCaptureStatus cst;
                 cudaGraph_t cg;
                 const cudaGraphNode_t *deps = nullptr;
@@ -1121,7 +1128,7 @@ template<class R> class Engine : public EngineBase {
                     break;
                 }
                 cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
-                cp.conditional.handle = hc;
+                cp.conditional.handle = hc[size_t(k)];
                 cp.conditional.type = cudaGraphCondTypeIf;
                 cp.conditional.size = 1;
                 cudaGraphNode_t cn;
@@ -1136,10 +1143,13 @@ template<class R> class Engine : public EngineBase {
                     break;
                 }
                 if (has_mesh) launch_mesh<R>(a, st);
-                if (P.integrator == ORBC_INT_NOSE_HOOVER)
+                if (nh) {
                     launch_nh_final<R>(a, st, P.energy != 0);
-                else
-                    launch_step_langevin<R>(a, st, P.energy != 0);
+                } else {
+                    ak.has_cond = k + 1 < steps_per_graph ? 1 : 0;
+                    if (ak.has_cond) ak.cond = hc[size_t(k) + 1];
+                    launch_step_langevin<R>(ak, st, P.energy != 0);
+                }
             }
             cudaGraph_t out = nullptr;
             cudaError_t e = cudaStreamEndCapture(st, &out);
@@ -1219,8 +1229,9 @@ template<class R> class Engine : public EngineBase {
         CK(cudaEventRecord(ev0, st));
         if (P.use_graph && nsteps > 0) {
             int k = 0;
-            for (; k + graph_steps <= nsteps; k += graph_steps) CK(cudaGraphLaunch(gexec, st));
-            for (; k < nsteps; ++k) CK(cudaGraphLaunch(gexec1, st));
+            const int64_t cond1 = graph_cond && P.integrator != ORBC_INT_NOSE_HOOVER ? 1 : 0;  // the condition kernel
+            for (; k + graph_steps <= nsteps; k += graph_steps, extra += cond1) CK(cudaGraphLaunch(gexec, st));
+            for (; k < nsteps; ++k, extra += cond1) CK(cudaGraphLaunch(gexec1, st));
         } else {
             for (int k = 0; k < nsteps; ++k) enqueue_step(true);
         }
@@ -1233,7 +1244,7 @@ template<class R> class Engine : public EngineBase {
         last_ms = ms;
         const Scalars before = hsc[0], hs = hsc[1];
         const int64_t nreb = hs.rebuilds - before.rebuilds;
-        const int per_step = P.use_graph && gexec ? fixed_launches_per_step() : (fixed_launches_per_step() - (graph_cond ? 1 : 0) + rebuild_launches());
+        const int per_step = P.use_graph && gexec ? fixed_launches_per_step() : (fixed_launches_per_step() + rebuild_launches());
         last_launches = extra + int64_t(nsteps) * per_step + (P.use_graph && graph_cond ? nreb * rebuild_launches() : 0);
         if (out) {
             int rc = thermo(-1, out);

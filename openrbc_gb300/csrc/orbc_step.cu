@@ -703,8 +703,9 @@ __device__ __forceinline__ void warp_partials(const KArgs<R> &a, int i, R ke, R 
     }
 }
 
+__device__ __forceinline__ double max_or_nan(double x, double y) { return (x > y || !(x == x)) ? x : y; }
 __device__ __forceinline__ double combine_part(int k, double x, double y) {
-    return k == 2 ? fmax(x, y) : (k == 3 ? double(int(x) | int(y)) : x + y);
+    return k == 2 ? max_or_nan(x, y) : (k == 3 ? double(int(x) | int(y)) : x + y);
 }
 
 /* Per-system sums, second and third level, after a kernel that wrote warp
@@ -715,7 +716,11 @@ __device__ __forceinline__ double combine_part(int k, double x, double y) {
  * thermostat, kinetic energy, potential energy, bulk velocity, rebuild rule,
  * step counter, buffer parity. */
 template<class R> __global__ void __launch_bounds__(RED_GROUP) k_reduce(KArgs<R> a, int mode, int count_step) {
-    if (halted(a.S)) return;  // the kernel before it did nothing; its partials are stale
+    if (halted(a.S)) {  // the kernel before it did nothing; its partials are stale
+        if (a.has_cond && blockIdx.x == 0 && threadIdx.x == 0)
+            cudaGraphSetConditional(a.cond, __ldcg(&a.S->rebuild) ? 1u : 0u);
+        return;
+    }
     __shared__ double red[7][RED_GROUP];
     __shared__ double wmax[RED_GROUP / 32];
     __shared__ int wfl[RED_GROUP / 32];
@@ -778,7 +783,7 @@ template<class R> __global__ void __launch_bounds__(RED_GROUP) k_reduce(KArgs<R>
                 ss.ke2 = k2;
                 if (mode == MODE_NH_FINAL) ss.epot = e;
             }
-            mymax = fmax(mymax, v[2]);
+            mymax = max_or_nan(v[2], mymax);
             myfl |= int(v[3]);
         }
     }
@@ -791,15 +796,17 @@ template<class R> __global__ void __launch_bounds__(RED_GROUP) k_reduce(KArgs<R>
         double m = 0.0;
         int fl = 0;
         for (int w = 0; w < RED_GROUP / 32; ++w) {
-            m = fmax(m, wmax[w]);
+            m = max_or_nan(wmax[w], m);
             fl |= wfl[w];
         }
         Scalars *S = a.S;
         S->error |= fl;
+        int rebuild = __ldcg(&S->rebuild);
         if (mode == MODE_LANGEVIN || mode == MODE_NH_INITIAL) {
             S->since_rebuild += 1;
-            if (m > double(a.skin_half2) || (a.rebuild_every > 0 && S->since_rebuild >= a.rebuild_every))
-                S->rebuild = 1;
+            // (a position that is not a number counts as moved: the build drops its particle)
+            if (!(m <= double(a.skin_half2)) || (a.rebuild_every > 0 && S->since_rebuild >= a.rebuild_every))
+                S->rebuild = rebuild = 1;
         }
         if (mode == MODE_LANGEVIN) {
             S->cur ^= 1;
@@ -815,6 +822,7 @@ template<class R> __global__ void __launch_bounds__(RED_GROUP) k_reduce(KArgs<R>
             }
         }
         S->blk_counter = 0;
+        if (a.has_cond) cudaGraphSetConditional(a.cond, rebuild ? 1u : 0u);
         __threadfence();
     }
 }
@@ -956,14 +964,19 @@ __global__ void __launch_bounds__(LITE_BS, force_blocks<R, K, U>()) k_step_lange
 
 /* After a lite Langevin step (count_step = 1) or a minimisation step (0):
  * flip the position buffers, advance the step counter and apply the
- * every-k-steps rebuild rule. */
-__global__ void k_advance(Scalars *S, int rebuild_every, int count_step) {
-    if (halted(S)) return;
-    S->iters += 1;
-    S->cur ^= 1;
-    S->step += count_step;
-    S->since_rebuild += 1;
-    if (rebuild_every > 0 && S->since_rebuild >= rebuild_every) S->rebuild = 1;
+ * every-k-steps rebuild rule; in a graph, hand the rebuild flag to the next
+ * step's conditional node (a kernel of its own for that cost 2 us a step). */
+__global__ void k_advance(Scalars *S, int rebuild_every, int count_step, cudaGraphConditionalHandle cond,
+                          int has_cond) {
+    int rebuild = __ldcg(&S->rebuild);
+    if (!halted(S)) {
+        S->iters += 1;
+        S->cur ^= 1;
+        S->step += count_step;
+        S->since_rebuild += 1;
+        if (rebuild_every > 0 && S->since_rebuild >= rebuild_every) S->rebuild = rebuild = 1;
+    }
+    if (has_cond) cudaGraphSetConditional(cond, rebuild ? 1u : 0u);
 }
 
 /* One step of the energy minimisation (src/openrbc.cpp:88-146): forces,
@@ -1359,7 +1372,7 @@ template<class R, bool K> void step_langevin_v(const KArgs<R> &a, cudaStream_t s
     if (energy || a.zero_bulk)
         reduce_sums<R>(a, MODE_LANGEVIN, 1, st);
     else
-        k_advance<<<1, 1, 0, st>>>(a.S, a.rebuild_every, 1);
+        k_advance<<<1, 1, 0, st>>>(a.S, a.rebuild_every, 1, a.cond, a.has_cond);
 }
 template<class R> void launch_step_langevin(const KArgs<R> &a, cudaStream_t st, bool energy) {
     if (a.kahan)
@@ -1410,7 +1423,7 @@ template<class R> void launch_minimize(const KArgs<R> &a, double dr_opt, double 
     by_batch<R>(a, [&](auto u, int nb) {
         k_minimize<R, decltype(u)::value><<<nb, LITE_BS, 0, st>>>(a, dr_opt, dn_opt);
     });
-    k_advance<<<1, 1, 0, st>>>(a.S, a.rebuild_every, 0);
+    k_advance<<<1, 1, 0, st>>>(a.S, a.rebuild_every, 0, a.cond, a.has_cond);
 }
 template<class R> void launch_vcom(const KArgs<R> &a, cudaStream_t st) {
     k_vcom<R><<<a.npad / 256, 256, 0, st>>>(a);
