@@ -80,43 +80,108 @@ template<class T> __global__ void __launch_bounds__(RDF_TILE) k_rdf(const typena
     const int ti = int(pi.w);
     const T dr = T(ra.dr), rcut = T(ra.rcut);
     const T L[3] = {T(ra.L[0]), T(ra.L[1]), T(ra.L[2])};
-    unsigned long long drop = 0;
+    unsigned drop = 0;
+    // one pair, every operation rounded as the oracle's
+    auto exact = [&](const T4 &q) {
+        T dd[3] = {o_sub(pi.x, q.x), o_sub(pi.y, q.y), o_sub(pi.z, q.z)};
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            if (L[d] > T(0)) dd[d] = o_sub(dd[d], o_mul(L[d], o_rint(o_div(dd[d], L[d]))));
+        const T r = o_sqrt(o_add(o_add(o_mul(dd[0], dd[0]), o_mul(dd[1], dd[1])), o_mul(dd[2], dd[2])));
+        if (rcut > T(0) && !(r < rcut)) {
+            ++drop;
+            return;
+        }
+        const T qb = o_div(r, dr);
+        const int b = qb < T(2147483647.0) ? int(qb) : 2147483647;
+        if (b >= ra.nbins)
+            ++drop;
+        else if (ra.smem_hist)
+            atomicAdd(&hist[b], 1u);
+        else
+            atomicAdd(&ra.counts[b], 1ull);
+    };
+    /* The same pair by an estimate of its distance.  On a periodic axis the
+     * image distance is min(t, L - t) of t = |dd| (t < 1.4 L, checked per
+     * tile), whichever side of the tie the rounded quotient falls; pairs within
+     * 1e-4 L of the tie are left to exact().  The estimate r is within 1e-6 of the
+     * rounded distance, so its bin is sure where r / dr (1 -+ 2e-6) agree, below
+     * the last bin and the cutoff (r_sure), and the pair is surely dropped
+     * beyond them (r_drop). */
+    const float dr_lo = float(1.0 / ra.dr) * (1.f - 2e-6f), dr_hi = float(1.0 / ra.dr) * (1.f + 2e-6f);
+    float r_end = float(ra.dr) * float(ra.nbins);
+    if (ra.rcut > 0) r_end = fminf(r_end, float(ra.rcut));
+    const float r_sure = r_end * (1.f - 3e-6f), r_drop = r_end * (1.f + 3e-6f);
+    T wide[3];  // no tie on an open axis: t - |L - t| with L = infinity
+    T Lx[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        Lx[d] = L[d] > T(0) ? L[d] : T(1e30);
+        wide[d] = L[d] > T(0) ? L[d] * T(2e-4) : T(0);
+    }
+    auto fast = [&](const T4 &q) {
+        const T dd[3] = {o_sub(pi.x, q.x), o_sub(pi.y, q.y), o_sub(pi.z, q.z)};
+        float m[3];
+        bool sure = true;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const T t = fabs(dd[d]), u = fabs(o_sub(Lx[d], t));
+            m[d] = float(t < u ? t : u);
+            sure = sure && fabs(t - u) > wide[d];
+        }
+        const float s2 = fmaf(m[2], m[2], fmaf(m[1], m[1], m[0] * m[0]));
+        float ri;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ri) : "f"(s2));
+        const float r = s2 * ri;  // not a number at distance 0
+        const int b = int(r * dr_lo);
+        if (sure && r < r_sure && b == int(r * dr_hi))
+            atomicAdd(&hist[b], 1u);
+        else if (sure && r > r_drop && r < 1e15f)
+            ++drop;
+        else
+            exact(q);
+    };
+    const bool typed = ra.ta >= 0 || ra.tb >= 0;
     for (int jt = max(jt0, it); jt < jt1; ++jt) {
         __syncthreads();
         const int jl = jt * RDF_TILE + threadIdx.x;
-        if (jl < ra.n) tile[threadIdx.x] = p[jl];
-        __syncthreads();
+        bool far = false;  // a coordinate beyond 0.7 L of the box's centre: t might pass 1.4 L
+        auto beyond = [&](const T4 &q) {
+            return (L[0] > T(0) && !(fabs(q.x) < T(0.7) * L[0])) || (L[1] > T(0) && !(fabs(q.y) < T(0.7) * L[1])) ||
+                   (L[2] > T(0) && !(fabs(q.z) < T(0.7) * L[2]));
+        };
+        if (jl < ra.n) {
+            tile[threadIdx.x] = p[jl];
+            far = beyond(tile[threadIdx.x]);
+        }
+        if (i < ra.n) far = far || beyond(pi);
+        far = __syncthreads_or(far || !ra.smem_hist || typed);
         if (i >= ra.n) continue;
         const int kend = min(RDF_TILE, ra.n - jt * RDF_TILE);
+        // neighbouring lanes start five apart in the tile: particles follow one
+        // another along rows, and 32 of them against one far particle would fall
+        // into the same few bins, whose additions the shared memory serialises
+        if (!far && jt != it && kend == RDF_TILE) {
+#pragma unroll 4
+            for (int k0 = 0; k0 < RDF_TILE; ++k0) fast(tile[(k0 + 5 * int(threadIdx.x)) & (RDF_TILE - 1)]);
+            continue;
+        }
         for (int k = (jt == it ? threadIdx.x + 1 : 0); k < kend; ++k) {
             const T4 q = tile[k];
             const int tj = int(q.w);
-            if (!((tmatch(ti, ra.ta) && tmatch(tj, ra.tb)) || (tmatch(ti, ra.tb) && tmatch(tj, ra.ta)))) continue;
-            T dd[3] = {o_sub(pi.x, q.x), o_sub(pi.y, q.y), o_sub(pi.z, q.z)};
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-                if (L[d] > T(0)) dd[d] = o_sub(dd[d], o_mul(L[d], o_rint(o_div(dd[d], L[d]))));
-            const T r = o_sqrt(o_add(o_add(o_mul(dd[0], dd[0]), o_mul(dd[1], dd[1])), o_mul(dd[2], dd[2])));
-            if (rcut > T(0) && !(r < rcut)) {
-                ++drop;
+            if (typed && !((tmatch(ti, ra.ta) && tmatch(tj, ra.tb)) || (tmatch(ti, ra.tb) && tmatch(tj, ra.ta))))
                 continue;
-            }
-            const T qb = o_div(r, dr);
-            const int b = qb < T(2147483647.0) ? int(qb) : 2147483647;
-            if (b >= ra.nbins) {
-                ++drop;
-                continue;
-            }
-            if (ra.smem_hist)
-                atomicAdd(&hist[b], 1u);
+            if (far)
+                exact(q);
             else
-                atomicAdd(&ra.counts[b], 1ull);
+                fast(q);
         }
     }
+    unsigned long long total_drop = drop;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) drop += __shfl_xor_sync(0xffffffffu, drop, o);
+    for (int o = 16; o > 0; o >>= 1) total_drop += __shfl_xor_sync(0xffffffffu, total_drop, o);
     __syncthreads();
-    if ((threadIdx.x & 31) == 0 && drop) atomicAdd(&sdrop, drop);
+    if ((threadIdx.x & 31) == 0 && total_drop) atomicAdd(&sdrop, total_drop);
     __syncthreads();
     if (threadIdx.x == 0 && sdrop) atomicAdd(ra.dropped, sdrop);
     if (ra.smem_hist)
