@@ -480,9 +480,9 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
     constexpr int NLW = 4;                                // warps per block
     constexpr int MB = 8;                                 // accept masks (32 candidates each) per lane
     constexpr int REG = 32 * MB;                          // candidates of one cell (or chunk) per phase 1
-    constexpr int SE = sizeof(T4) == 16 ? 768 : 512;      // list entries staged per warp until phase 2
+    constexpr int SE = 768;                               // list entries staged per warp until phase 2
     __shared__ float2 s_cut[256];                         // (list cutoff^2, inner cutoff^2) per type pair
-    __shared__ T4 s_pos[NLW][REG];                        // the current cell's candidates
+    __shared__ float4 s_pos[NLW][REG];                    // the current cell's candidates (FP64: rounded)
     __shared__ uint32_t s_ent[NLW][SE];                   // j | shift code of its cell << NB_SHIFT
     __shared__ int s_off[NLW][28], s_beg[NLW][27];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -514,10 +514,36 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
         const R ex = pi.x - qs.x, ey = pi.y - qs.y, ez = pi.z - qs.z;
         return ex * ex + ey * ey + ez * ez;
     };
+    // FP64: the two comparisons of a test are decided in FP32 (from rounded
+    // positions) unless r^2 lies within the rounding of a cutoff for some lane;
+    // coordinates up to 2 Lc rounded to 2^-24 of it move r^2 by 5e-7 Lc near the
+    // cutoffs.  Half a million FP64 tests per thousand particles otherwise bound
+    // the build: 250 thousand particle cell 0.84 -> 0.28 ms
+    const float slack = 1e-5f + 8e-6f * fmaxf(sd.Lcf[0], fmaxf(sd.Lcf[1], sd.Lcf[2]));
+    // ballots of r^2 < cut.x, cut.y for candidate q of lane; et: its list entry (FP64)
+    auto inside = [&](const T4 &pi, const float4 &pf, const float4 &q, const float2 &cut, const uint32_t *et, bool pad,
+                      unsigned &ma, unsigned &mi) {
+        const float ex = pf.x - q.x, ey = pf.y - q.y, ez = pf.z - q.z;
+        const float r2 = ex * ex + ey * ey + ez * ez;
+        ma = __ballot_sync(0xffffffffu, r2 < cut.x);
+        mi = __ballot_sync(0xffffffffu, r2 < cut.y);
+        if constexpr (sizeof(R) == 8) {
+            const bool near = fabsf(r2 - cut.x) < slack * cut.x || fabsf(r2 - cut.y) < slack * cut.y;
+            if (__any_sync(0xffffffffu, near)) {
+                R d2 = R(1e30);
+                if (!pad) {
+                    const int l = int(*et >> NB_SHIFT);
+                    d2 = dist2(pi, shifted(a.pos[cur][*et & NB_MASK], l % 3 - 1, (l / 3) % 3 - 1, l / 9 - 1));
+                }
+                ma = __ballot_sync(0xffffffffu, d2 < R(cut.x));
+                mi = __ballot_sync(0xffffffffu, d2 < R(cut.y));
+            }
+        }
+    };
     const int kme = cc[0] | (cc[1] << 11) | (cc[2] << 22);
     int *off = s_off[warp];
     int *beg = s_beg[warp];
-    T4 *sp = s_pos[warp];
+    float4 *sp = s_pos[warp];
     uint32_t *se = s_ent[warp];
     uint32_t *col = a.nbr + nbr_index(i, 0, a.cap);  // row k of slot i at col[32 k]
     const int cap = a.cap;
@@ -565,15 +591,18 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
                 if (l + step < 27 && off[l + step] <= idx) l += step;
             const int j = beg[l] + (idx - off[l]);
             const T4 q = a.pos[cur][j];
-            types |= w_type(wbits(q.w));
-            sp[t] = shifted(q, l % 3 - 1, (l / 3) % 3 - 1, l / 9 - 1);
+            const int tj = w_type(wbits(q.w));
+            types |= tj;
+            if constexpr (sizeof(R) == 4)
+                sp[t] = shifted(q, l % 3 - 1, (l / 3) % 3 - 1, l / 9 - 1);
+            else
+                sp[t] = make_float4(float(q.x) + float(l % 3 - 1) * sd.Lcf[0],
+                                    float(q.y) + float((l / 3) % 3 - 1) * sd.Lcf[1],
+                                    float(q.z) + float(l / 9 - 1) * sd.Lcf[2], __int_as_float(tj));
             se[ebase + t] = uint32_t(j) | (uint32_t(l) << NB_SHIFT);
         }
         if (nch + lane < ((nch + 31) & ~31)) {  // far away: never accepted
-            T4 z;
-            z.x = z.y = z.z = R(1e18);
-            z.w = R(0);
-            sp[nch + lane] = z;
+            sp[nch + lane] = make_float4(1e18f, 1e18f, 1e18f, 0.f);
         }
         __syncwarp();
         return __reduce_or_sync(0xffffffffu, types);
@@ -581,7 +610,7 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
     uint32_t macc[MB], minn[MB];
     // phase 1 for the particles grp, two per pass, over the staged candidates [0, nch), nch <= REG.
     // ONE: one list and one inner cutoff; otherwise cutoffs by type pair
-    auto phase1 = [&](unsigned grp, int nch, auto one_cutoff) {
+    auto phase1 = [&](unsigned grp, int nch, int ebase, auto one_cutoff) {
         constexpr bool ONE = decltype(one_cutoff)::value;
         for (unsigned g = grp; g;) {
             const int il = __ffs(int(g)) - 1;
@@ -595,22 +624,23 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
             pi2.x = __shfl_sync(0xffffffffu, p.x, il2);
             pi2.y = __shfl_sync(0xffffffffu, p.y, il2);
             pi2.z = __shfl_sync(0xffffffffu, p.z, il2);
+            const float4 pf = make_float4(float(pi.x), float(pi.y), float(pi.z), 0.f),
+                         pf2 = make_float4(float(pi2.x), float(pi2.y), float(pi2.z), 0.f);
             const int ti = ONE ? 0 : __shfl_sync(0xffffffffu, ty, il) * 16;
             const int ti2 = ONE ? 0 : __shfl_sync(0xffffffffu, ty, il2) * 16;
 #pragma unroll
             for (int b = 0; b < MB; ++b) {
                 if (b * 32 < nch) {
-                    const T4 q = sp[b * 32 + lane];
+                    const float4 q = sp[b * 32 + lane];
                     const int tj = ONE ? 0 : w_type(wbits(q.w));
+                    const uint32_t *et = se + ebase + b * 32 + lane;
+                    const bool pad = b * 32 + lane >= nch;
                     const float2 cut = ONE ? cut_ll : s_cut[ti + tj];
                     const float2 cut2 = ONE ? cut_ll : s_cut[ti2 + tj];
-                    const R r2 = dist2(pi, q);
-                    const R r2b = dist2(pi2, q);
                     // inner cutoff <= list cutoff; a particle's own bit is cleared in phase 2
-                    const unsigned ma = __ballot_sync(0xffffffffu, r2 < R(cut.x));
-                    unsigned mi = __ballot_sync(0xffffffffu, r2 < R(cut.y));
-                    const unsigned ma2 = __ballot_sync(0xffffffffu, r2b < R(cut2.x));
-                    unsigned mi2 = __ballot_sync(0xffffffffu, r2b < R(cut2.y));
+                    unsigned ma, mi, ma2, mi2;
+                    inside(pi, pf, q, cut, et, pad, ma, mi);
+                    inside(pi2, pf2, q, cut2, et, pad, ma2, mi2);
                     if (lane == il) {
                         macc[b] = ma;
                         minn[b] = mi;
@@ -675,10 +705,10 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
         myself = -1;
         __syncwarp();  // every lane is done with se before it is restaged
     };
-    auto test = [&](unsigned grp, int nch, unsigned types) {
+    auto test = [&](unsigned grp, int nch, int ebase, unsigned types) {
         types |= __reduce_or_sync(0xffffffffu, (grp >> lane) & 1u ? unsigned(ty) : 0u);
         if (types < 4u && a.uniform_cut) {
-            phase1(grp, nch, std::true_type());
+            phase1(grp, nch, ebase, std::true_type());
             if (types) {  // the inner partners of types 0..3 are the lipids
 #pragma unroll
                 for (int b = 0; b < MB; ++b) {
@@ -689,7 +719,7 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
                 }
             }
         } else {
-            phase1(grp, nch, std::false_type());
+            phase1(grp, nch, ebase, std::false_type());
         }
     };
 #pragma unroll
@@ -711,7 +741,7 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
             mybase = 0;
             for (int c0 = 0; c0 < total_c; c0 += REG) {
                 const int nch = min(REG, total_c - c0);
-                test(grp, nch, stage(c0, nch, 0));
+                test(grp, nch, 0, stage(c0, nch, 0));
                 if (member) myself = (ts >= c0 && ts < c0 + nch) ? ts - c0 : -1;
                 phase2();
             }
@@ -722,7 +752,7 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
             pend = 0u;
             eused = 0;
         }
-        test(grp, total_c, stage(0, total_c, eused));
+        test(grp, total_c, eused, stage(0, total_c, eused));
         if (member) {
             mybase = eused;
             myself = ts;

@@ -235,14 +235,39 @@ template<class R> __device__ __forceinline__ void kahan_add(R &s, R &c, R d) {
 template<class R> struct ShiftTab {
     R v[3][32];
 };
+template<> struct ShiftTab<double> {
+    double v[3][32];
+    float f[3][32];  // rounded, for the shell test
+    float slack;     // relative error bound of the rounded test
+};
 template<class R> __device__ __forceinline__ void init_shift(const SysDev &sd, ShiftTab<R> &sh) {
     const int lane = threadIdx.x & 31;
     if (lane < 27) {
         sh.v[0][lane] = R(-(lane % 3 - 1)) * lc_of<R>(sd, 0);
         sh.v[1][lane] = R(-((lane / 3) % 3 - 1)) * lc_of<R>(sd, 1);
         sh.v[2][lane] = R(-(lane / 9 - 1)) * lc_of<R>(sd, 2);
+        if constexpr (sizeof(R) == 8)
+            for (int d = 0; d < 3; ++d) sh.f[d][lane] = float(sh.v[d][lane]);
+        // coordinates up to Lc, rounded to 2^-24 of it, put 2.4e-7 Lc of relative error into r^2 near the cutoffs
+        if constexpr (sizeof(R) == 8)
+            if (lane == 0) sh.slack = 1e-5f + 4e-6f * fmaxf(sd.Lcf[0], fmaxf(sd.Lcf[1], sd.Lcf[2]));
     }
     __syncwarp();
+}
+/* Whether the pair of a shell row is inside r^2 < lim, for the FP64 form: in
+ * FP32 where the rounding of the coordinates cannot change the answer, and
+ * by the FP64 distance in the thin shell that remains. */
+__device__ __forceinline__ bool shell_inside(const ShiftTab<double> &sh, const double4a &pi, const double4a &pj, int c,
+                                             double lim) {
+    const float fx = float(pi.x) - float(pj.x) + sh.f[0][c], fy = float(pi.y) - float(pj.y) + sh.f[1][c],
+                fz = float(pi.z) - float(pj.z) + sh.f[2][c];
+    const float r2 = fx * fx + fy * fy + fz * fz, l = float(lim);
+    if (r2 < l * (1.f - sh.slack)) return true;
+    if (r2 > l * (1.f + sh.slack)) return false;
+    const double dx = __dadd_rn(__dadd_rn(pi.x, -pj.x), sh.v[0][c]);
+    const double dy = __dadd_rn(__dadd_rn(pi.y, -pj.y), sh.v[1][c]);
+    const double dz = __dadd_rn(__dadd_rn(pi.z, -pj.z), sh.v[2][c]);
+    return __fma_rn(dz, dz, __fma_rn(dy, dy, __dmul_rn(dx, dx))) < lim;
 }
 
 /* ------------------------------------------------------------------------- */
@@ -269,6 +294,17 @@ __device__ __forceinline__ double rsqrt_pair(double r2) {
     const double e = fma_rn(-mul_rn(r2, y), y, 1.0);
     return fma_rn(mul_rn(fma_rn(e, 0.375, 0.5), e), y, y);
 }
+
+/* r2 > 1e-5 and max(x, 0).  In FP64 on the integer pipe, as an FP64 comparison
+ * takes as long as a multiplication there: numbers above a positive one
+ * compare as their bits do (infinity included, the NaNs above it not). */
+__device__ __forceinline__ bool apart(float r2) { return r2 > 1e-5f; }
+__device__ __forceinline__ bool apart(double r2) {
+    const long long b = __double_as_longlong(r2);
+    return b > __double_as_longlong(1e-5) && b <= 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ float positive_part(float x) { return fmaxf(x, 0.f); }
+__device__ __forceinline__ double positive_part(double x) { return __double2hiint(x) < 0 ? 0.0 : x; }
 
 /* The anisotropic pair with a lipid j, by the owner's own parameters, in the
  * form that keeps the neighbour's vectors outermost:
@@ -307,9 +343,9 @@ template<class R, bool E, bool K>
 __device__ __forceinline__ void pair_term(PairAcc<R, K> &A, const OwnP<R> &P, const R d[3], const R n[3], R nix, R niy,
                                           R niz) {
     const R r2 = fma_rn(d[2], d[2], fma_rn(d[1], d[1], mul_rn(d[0], d[0])));
-    const R r2c = r2 > R(1e-5) ? r2 : R(1e30);  // coinciding particles: no force, as outside the range
+    const R r2c = apart(r2) ? r2 : R(1e30);  // coinciding particles: no force, as outside the range
     const R ri = rsqrt_pair(r2c);
-    const R rc = max(fma_rn(-r2c, ri, P.cut), R(0));
+    const R rc = positive_part(fma_rn(-r2c, ri, P.cut));
     const R nn = fma_rn(niz, n[2], fma_rn(niy, n[1], mul_rn(nix, n[0])));
     const R niu = mul_rn(fma_rn(niz, d[2], fma_rn(niy, d[1], mul_rn(nix, d[0]))), ri);
     const R nju = mul_rn(fma_rn(n[2], d[2], fma_rn(n[1], d[1], mul_rn(n[0], d[0]))), ri);
@@ -409,9 +445,14 @@ __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, 
             for (int u = 0; u < SHELL_U; ++u) pj[u] = ldg4<R>(pos + (ent[u] & NB_MASK));
 #pragma unroll
             for (int u = 0; u < SHELL_U; ++u) {
-                R d[3];
-                offset(ent[u], pj[u], d);
-                if (k + u < nq && dist2(d) < lim) hm |= 1u << (k + u);
+                if constexpr (sizeof(R) == 8) {
+                    const bool in = shell_inside(sh, pi, pj[u], int(ent[u] >> NB_SHIFT), lim);
+                    if (k + u < nq && in) hm |= 1u << (k + u);
+                } else {
+                    R d[3];
+                    offset(ent[u], pj[u], d);
+                    if (k + u < nq && dist2(d) < lim) hm |= 1u << (k + u);
+                }
             }
         }
         const int total = int(__reduce_max_sync(0xffffffffu, unsigned(nin + __popc(hm))));
