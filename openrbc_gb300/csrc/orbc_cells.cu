@@ -480,11 +480,13 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
     constexpr int NLW = 4;                                // warps per block
     constexpr int MB = 8;                                 // accept masks (32 candidates each) per lane
     constexpr int REG = 32 * MB;                          // candidates of one cell (or chunk) per phase 1
+    constexpr int SU = 2;                                 // blocks of 32 candidates staged together
     constexpr int SE = 768;                               // list entries staged per warp until phase 2
     __shared__ float2 s_cut[256];                         // (list cutoff^2, inner cutoff^2) per type pair
     __shared__ float4 s_pos[NLW][REG];                    // the current cell's candidates (FP64: rounded)
     __shared__ uint32_t s_ent[NLW][SE];                   // j | shift code of its cell << NB_SHIFT
-    __shared__ int s_off[NLW][28], s_beg[NLW][27];
+    __shared__ float4 s_seg[NLW][27];                     // occupied neighbour cells: shift, first slot - first candidate
+    __shared__ uint32_t s_code[NLW][27];                  // and their shift code << NB_SHIFT
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int k = threadIdx.x; k < 256; k += blockDim.x)
         s_cut[k] = make_float2(__ldg(&a.ff->rlist2[k]), __ldg(&a.ff->rin2[k]));
@@ -541,15 +543,17 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
         }
     };
     const int kme = cc[0] | (cc[1] << 11) | (cc[2] << 22);
-    int *off = s_off[warp];
-    int *beg = s_beg[warp];
+    float4 *seg = s_seg[warp];
+    uint32_t *code = s_code[warp];
     float4 *sp = s_pos[warp];
     uint32_t *se = s_ent[warp];
     uint32_t *col = a.nbr + nbr_index(i, 0, a.cap);  // row k of slot i at col[32 k]
     const int cap = a.cap;
     const float2 cut_ll = s_cut[0];
     int qin = 0, qout = 0, qtot = 0;
-    // neighbour ranges of cell kd -> off/beg; returns the candidate count
+    // neighbour ranges of cell kd: this lane's candidates [first, first + cnt) of the cell's; the occupied
+    // cells' table; returns the candidate count.  own_first: where the centre cell's candidates begin
+    int first = 0, cnt = 0, own_first = 0, own_slot = 0;
     auto fetch = [&](int kd) {
         const int xd = kd & 2047, yd = (kd >> 11) & 2047, zd = (kd >> 22) & 1023;
         int2 rg = make_int2(0, 0);
@@ -564,42 +568,63 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
             else ok = ok && z >= 0 && z < sd.nc[2];
             if (ok) rg = a.ranges[sd.cell_base + cell_code(sd, x, y, z)];
         }
-        const int cnt = rg.y > rg.x ? rg.y - rg.x : 0;
+        cnt = rg.y > rg.x ? rg.y - rg.x : 0;
         int inc = cnt;  // inclusive warp scan
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int t = __shfl_up_sync(0xffffffffu, inc, o);
             if (lane >= o) inc += t;
         }
-        __syncwarp();  // the previous cell's staging is done with off/beg
-        if (lane < 27) {
-            off[lane] = inc - cnt;
-            beg[lane] = rg.x;
+        first = inc - cnt;
+        own_first = __shfl_sync(0xffffffffu, first, 13);
+        own_slot = __shfl_sync(0xffffffffu, rg.x, 13);
+        const unsigned occ = __ballot_sync(0xffffffffu, cnt > 0);
+        __syncwarp();  // the previous cell's staging is done with the table
+        if (cnt > 0) {
+            const int r = __popc(occ & ((1u << lane) - 1u));
+            seg[r] = make_float4(float(lane % 3 - 1) * sd.Lcf[0], float((lane / 3) % 3 - 1) * sd.Lcf[1],
+                                 float(lane / 9 - 1) * sd.Lcf[2], __int_as_float(rg.x - first));
+            code[r] = uint32_t(lane) << NB_SHIFT;
         }
         __syncwarp();
         return __shfl_sync(0xffffffffu, inc, 31);
     };
     // candidates [c0, c0 + nch) of the fetched cell -> sp[0 ...] and se[ebase ...]; the or of their types
+    // (c0 a multiple of 32).  A candidate's cell is the number of occupied cells that begin at or before it: a
+    // population count on the mask of beginnings in its block of 32, where a search over the 27 offsets
+    // takes five dependent lookups
     auto stage = [&](int c0, int nch, int ebase) {
         unsigned types = 0;
-#pragma unroll 4
-        for (int t = lane; t < nch; t += 32) {
-            const int idx = c0 + t;
-            int l = 0;  // last neighbour cell with off[l] <= idx
+        int before = __popc(__ballot_sync(0xffffffffu, cnt > 0 && first < c0));
+        for (int t0 = 0; t0 < nch; t0 += 32 * SU) {
+            int r[SU], j[SU];
+            float4 g[SU];
+            T4 q[SU];
 #pragma unroll
-            for (int step = 16; step > 0; step >>= 1)
-                if (l + step < 27 && off[l + step] <= idx) l += step;
-            const int j = beg[l] + (idx - off[l]);
-            const T4 q = a.pos[cur][j];
-            const int tj = w_type(wbits(q.w));
-            types |= tj;
-            if constexpr (sizeof(R) == 4)
-                sp[t] = shifted(q, l % 3 - 1, (l / 3) % 3 - 1, l / 9 - 1);
-            else
-                sp[t] = make_float4(float(q.x) + float(l % 3 - 1) * sd.Lcf[0],
-                                    float(q.y) + float((l / 3) % 3 - 1) * sd.Lcf[1],
-                                    float(q.z) + float(l / 9 - 1) * sd.Lcf[2], __int_as_float(tj));
-            se[ebase + t] = uint32_t(j) | (uint32_t(l) << NB_SHIFT);
+            for (int u = 0; u < SU; ++u) {
+                const int b = (t0 >> 5) + u;
+                const unsigned begins =
+                    __reduce_or_sync(0xffffffffu, cnt > 0 && (first - c0) >> 5 == b ? 1u << (first & 31) : 0u);
+                r[u] = before + __popc(begins & (0xffffffffu >> (31 - lane))) - 1;
+                before += __popc(begins);
+            }
+#pragma unroll
+            for (int u = 0; u < SU; ++u) {  // every load of the batch before its first store
+                g[u] = seg[r[u]];
+                j[u] = t0 + 32 * u + lane < nch ? c0 + t0 + 32 * u + lane + __float_as_int(g[u].w) : i;
+                q[u] = a.pos[cur][j[u]];
+            }
+#pragma unroll
+            for (int u = 0; u < SU; ++u) {
+                const int t = t0 + 32 * u + lane;
+                if (t < nch) {
+                    const int tj = w_type(wbits(q[u].w));
+                    types |= tj;
+                    sp[t] = make_float4(float(q[u].x) + g[u].x, float(q[u].y) + g[u].y, float(q[u].z) + g[u].z,
+                                        __int_as_float(tj));
+                    se[ebase + t] = uint32_t(j[u]) | code[r[u]];
+                }
+            }
         }
         if (nch + lane < ((nch + 31) & ~31)) {  // far away: never accepted
             sp[nch + lane] = make_float4(1e18f, 1e18f, 1e18f, 0.f);
@@ -732,7 +757,7 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
         const unsigned grp = __ballot_sync(0xffffffffu, real && kme == kd) & todo;
         const int total_c = fetch(kd);
         todo &= ~grp;
-        const int ts = off[13] + (i - beg[13]);
+        const int ts = own_first + (i - own_slot);
         const bool member = (grp >> lane) & 1u;
         if (total_c > REG) {  // in chunks of REG, each placed at once
             if (pend) phase2();
