@@ -248,6 +248,7 @@ template<class R> void launch_nh_initial(const KArgs<R> &a, cudaStream_t st);
 template<class R> void launch_nh_prologue(const KArgs<R> &a, cudaStream_t st);
 template<class R> void launch_forces(const KArgs<R> &a, cudaStream_t st);
 template<class R> void launch_vcom(const KArgs<R> &a, cudaStream_t st);
+template<class R> void launch_count_general(const KArgs<R> &a, unsigned long long *out, cudaStream_t st);
 template<class R> void launch_minimize(const KArgs<R> &a, double dr_opt, double dn_opt, cudaStream_t st);
 template<class R>
 void launch_frame_pack(const KArgs<R> &a, const int *file_of_home, int real_bytes, void *pos, void *vel, void *rot,

@@ -1593,6 +1593,17 @@ template<class R> class Engine : public EngineBase {
                 tin += hn[size_t(p)] & 0xffff;
                 ++cnt;
             }
+        // general pairs are listed in the shell rows whatever their distance
+        DevBuf<unsigned long long> ngen;
+        unsigned long long hgen = 0;
+        CK(ngen.alloc(1));
+        CK(cudaMemcpyAsync(ngen.p, &hgen, sizeof(hgen), cudaMemcpyHostToDevice, st));
+        launch_count_general<R>(a, ngen.p, st);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(&hgen, ngen.p, sizeof(hgen), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        ngen.release();
+        tin += double(hgen);
         out->mean_neighbors = cnt ? tot / double(cnt) : 0.0;
         out->pairs_in_cutoff = cnt ? tin / double(cnt) : 0.0;  // inner entries at the last build
         return ORBC_OK;

@@ -1291,6 +1291,32 @@ __global__ void __launch_bounds__(LITE_BS, force_blocks<R, true, U>()) k_forces(
     warp_partials<R>(a, i, R(0), e, 0.f, flags);
 }
 
+/* Shell entries of the general pairs (those the build puts there whatever
+ * their distance) that were inside their range when the list was built: with
+ * the inner entries, the partners in range (profile). */
+template<class R> __global__ void __launch_bounds__(256) k_count_general(KArgs<R> a, unsigned long long *out) {
+    using T4 = typename Vec<R>::T4;
+    const int lp = __ldcg(&a.S->lp);
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    const SysDev &sd = a.sys[a.blk_sys[i / SYS_PAD]];
+    const T4 p = a.xref[lp][i];
+    const int ty = w_type(wbits(p.w));
+    const int nout = ty != GHOST ? a.nnb[i] >> 16 : 0;
+    unsigned c = 0;
+    for (int k = 0; k < nout; ++k) {
+        const uint32_t ent = a.nbr[nbr_index(i, a.cap - 1 - k, a.cap)];
+        const T4 q = a.xref[lp][ent & NB_MASK];
+        const int tj = w_type(wbits(q.w)), s = int(ent >> NB_SHIFT);
+        const PairP<R> &P = a.ff->pair[ty * NT + tj];
+        if (tj == 0 && P.kind == PAIR_ANISO) continue;
+        const R dx = p.x - q.x - R(s % 3 - 1) * lc_of<R>(sd, 0), dy = p.y - q.y - R((s / 3) % 3 - 1) * lc_of<R>(sd, 1),
+                dz = p.z - q.z - R(s / 9 - 1) * lc_of<R>(sd, 2);
+        c += dx * dx + dy * dy + dz * dz < P.anysq ? 1u : 0u;
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, (unsigned long long)c);
+}
+
 /* FP64 membrane area and enclosed volume of each system's face mesh, and
  * the constraint coefficients for the next force evaluation.  Each block sums
  * MESH_CHUNK faces of one system; the last block adds the block sums of each
@@ -1466,6 +1492,9 @@ template<class R> void launch_minimize(const KArgs<R> &a, double dr_opt, double 
     });
     k_advance<<<1, 1, 0, st>>>(a.S, a.rebuild_every, 0, a.cond, a.has_cond);
 }
+template<class R> void launch_count_general(const KArgs<R> &a, unsigned long long *out, cudaStream_t st) {
+    k_count_general<R><<<a.npad / 256, 256, 0, st>>>(a, out);
+}
 template<class R> void launch_vcom(const KArgs<R> &a, cudaStream_t st) {
     k_vcom<R><<<a.npad / 256, 256, 0, st>>>(a);
     reduce_sums<R>(a, MODE_VCOM, 0, st);
@@ -1481,6 +1510,7 @@ template<class R> void launch_assign_temperature(const KArgs<R> &a, double kT, u
     template void launch_nh_initial<R>(const KArgs<R> &, cudaStream_t);               \
     template void launch_forces<R>(const KArgs<R> &, cudaStream_t);                   \
     template void launch_vcom<R>(const KArgs<R> &, cudaStream_t);                     \
+    template void launch_count_general<R>(const KArgs<R> &, unsigned long long *, cudaStream_t); \
     template void launch_minimize<R>(const KArgs<R> &, double, double, cudaStream_t); \
     template void launch_assign_temperature<R>(const KArgs<R> &, double, uint64_t, cudaStream_t); \
     template void launch_mesh<R>(const KArgs<R> &, cudaStream_t);
