@@ -474,23 +474,21 @@ template<class R> __device__ __forceinline__ void nlist_finalise(const KArgs<R> 
 // the cell with anchors slower (0.379 ms: the instruction cache).
 // 7 resident blocks per SM: the staging below (about 31 KB per block in FP32)
 // and at most 72 registers; more warps in flight beat fewer passes per warp
-template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArgs<R> a, int gated) {
+constexpr int NLW = 2;  // warps per block of the list build
+template<class R, int SW> __global__ void __launch_bounds__(32 * NLW, 28 / NLW) k_nlist(KArgs<R> a, int gated) {
     using T4 = typename Vec<R>::T4;
     if (gated && !__ldcg(&a.S->rebuild)) return;
-    constexpr int NLW = 4;                                // warps per block
     constexpr int MB = 8;                                 // accept masks (32 candidates each) per lane
     constexpr int REG = 32 * MB;                          // candidates of one cell (or chunk) per phase 1
     constexpr int SU = 2;                                 // blocks of 32 candidates staged together
-    constexpr int SE = 768;                               // list entries staged per warp until phase 2
-    __shared__ float2 s_cut[256];                         // (list cutoff^2, inner cutoff^2) per type pair
+    constexpr int SE = 704;                               // list entries staged per warp until phase 2
     __shared__ float4 s_pos[NLW][REG];                    // the current cell's candidates (FP64: rounded)
     __shared__ uint32_t s_ent[NLW][SE];                   // j | shift code of its cell << NB_SHIFT
     __shared__ float4 s_seg[NLW][27];                     // occupied neighbour cells: shift, first slot - first candidate
     __shared__ uint32_t s_code[NLW][27];                  // and their shift code << NB_SHIFT
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int k = threadIdx.x; k < 256; k += blockDim.x)
-        s_cut[k] = make_float2(__ldg(&a.ff->rlist2[k]), __ldg(&a.ff->rin2[k]));
-    __syncthreads();
+    // (list cutoff^2, inner cutoff^2) of a type pair
+    auto cuts = [&](int k) { return make_float2(__ldg(&a.ff->rlist2[k]), __ldg(&a.ff->rin2[k])); };
     const int cur = 1 - __ldcg(&a.S->cur), lp = 1 - __ldcg(&a.S->lp);
     // the grid covers npad (a multiple of the block size) SW times
     const int wid = blockIdx.x * NLW + warp;
@@ -549,7 +547,7 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
     uint32_t *se = s_ent[warp];
     uint32_t *col = a.nbr + nbr_index(i, 0, a.cap);  // row k of slot i at col[32 k]
     const int cap = a.cap;
-    const float2 cut_ll = s_cut[0];
+    const float2 cut_ll = cuts(0);
     int qin = 0, qout = 0, qtot = 0;
     // neighbour ranges of cell kd: this lane's candidates [first, first + cnt) of the cell's; the occupied
     // cells' table; returns the candidate count.  own_first: where the centre cell's candidates begin
@@ -660,8 +658,8 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
                     const int tj = ONE ? 0 : w_type(wbits(q.w));
                     const uint32_t *et = se + ebase + b * 32 + lane;
                     const bool pad = b * 32 + lane >= nch;
-                    const float2 cut = ONE ? cut_ll : s_cut[ti + tj];
-                    const float2 cut2 = ONE ? cut_ll : s_cut[ti2 + tj];
+                    const float2 cut = ONE ? cut_ll : cuts(ti + tj);
+                    const float2 cut2 = ONE ? cut_ll : cuts(ti2 + tj);
                     // inner cutoff <= list cutoff; a particle's own bit is cleared in phase 2
                     unsigned ma, mi, ma2, mi2;
                     inside(pi, pf, q, cut, et, pad, ma, mi);
@@ -796,11 +794,11 @@ template<class R, int SW> __global__ void __launch_bounds__(128, 7) k_nlist(KArg
 template<class R> void launch_nlist(const KArgs<R> &a, cudaStream_t st, int gated) {
     const int nw = a.npad / 32, room = 152 * 28;  // nw is a multiple of 8
     if (nw * 4 <= room)
-        k_nlist<R, 4><<<nw, 128, 0, st>>>(a, gated);
+        k_nlist<R, 4><<<nw * 4 / NLW, 32 * NLW, 0, st>>>(a, gated);
     else if (nw * 2 <= room)
-        k_nlist<R, 2><<<nw / 2, 128, 0, st>>>(a, gated);
+        k_nlist<R, 2><<<nw * 2 / NLW, 32 * NLW, 0, st>>>(a, gated);
     else
-        k_nlist<R, 1><<<nw / 4, 128, 0, st>>>(a, gated);
+        k_nlist<R, 1><<<nw / NLW, 32 * NLW, 0, st>>>(a, gated);
 }
 
 static int grid_for(int64_t n, int per_block = 256) {
