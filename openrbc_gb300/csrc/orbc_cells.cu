@@ -467,15 +467,17 @@ template<class R> __device__ __forceinline__ void nlist_finalise(const KArgs<R> 
  * SW warps share 32 slots, each taking 32 / SW of their particles: one warp's
  * chain of cells, ballots and expansions is some 80 thousand cycles long, which
  * is the time of the build while the GPU is not full. */
-// Bound by instruction issue (70 % of peak, 9.0 thousand warp instructions per
-// 32 slots, half of them cell ranges and staging).  1.0M-particle cell 0.357 ->
-// 0.348 ms, 1.0M lipids in 23 vesicles 0.359 -> 0.332 ms against table lookups
-// and a single expansion loop; a third copy of phase 1 for lipids alone made
-// the cell with anchors slower (0.379 ms: the instruction cache).
-// 7 resident blocks per SM: the staging below (about 31 KB per block in FP32)
-// and at most 72 registers; more warps in flight beat fewer passes per warp
+// Bound by instruction issue (61 % of peak) and each warp's chain.  1.0M-particle
+// cell 0.357 -> 0.266 ms, 4.03M 1.34 -> 0.98, 1.0M lipids in 23 vesicles 0.359 ->
+// 0.279 against table lookups, searched staging and blocks of four warps; a third
+// copy of phase 1 for lipids alone made the cell with anchors slower (0.379 ms:
+// the instruction cache).
+// 28 resident warps per SM: the staging below (about 15 KB per block) and at
+// most 72 registers (FP64: 24 and 80, where 72 spill); more warps in flight beat
+// fewer passes per warp.  Blocks of two warps: one of four holds its memory until
+// its slowest warp is done (4.03M 1.08 ms), single warps fit only 26 (1.10 ms).
 constexpr int NLW = 2;  // warps per block of the list build
-template<class R, int SW> __global__ void __launch_bounds__(32 * NLW, 28 / NLW) k_nlist(KArgs<R> a, int gated) {
+template<class R, int SW> __global__ void __launch_bounds__(32 * NLW, (sizeof(R) == 8 ? 24 : 28) / NLW) k_nlist(KArgs<R> a, int gated) {
     using T4 = typename Vec<R>::T4;
     if (gated && !__ldcg(&a.S->rebuild)) return;
     constexpr int MB = 8;                                 // accept masks (32 candidates each) per lane
@@ -517,8 +519,7 @@ template<class R, int SW> __global__ void __launch_bounds__(32 * NLW, 28 / NLW) 
     // FP64: the two comparisons of a test are decided in FP32 (from rounded
     // positions) unless r^2 lies within the rounding of a cutoff for some lane;
     // coordinates up to 2 Lc rounded to 2^-24 of it move r^2 by 5e-7 Lc near the
-    // cutoffs.  Half a million FP64 tests per thousand particles otherwise bound
-    // the build: 250 thousand particle cell 0.84 -> 0.28 ms
+    // cutoffs.  Some 124 FP64 tests per particle otherwise bound the build: 250 thousand particle cell 0.84 -> 0.15 ms
     const float slack = 1e-5f + 8e-6f * fmaxf(sd.Lcf[0], fmaxf(sd.Lcf[1], sd.Lcf[2]));
     // ballots of r^2 < cut.x, cut.y for candidate q of lane; et: its list entry (FP64)
     auto inside = [&](const T4 &pi, const float4 &pf, const float4 &q, const float2 &cut, const uint32_t *et, bool pad,
@@ -790,7 +791,8 @@ template<class R, int SW> __global__ void __launch_bounds__(32 * NLW, 28 / NLW) 
 
 /* As many warps per 32 slots (4, 2 or 1) as are all resident at once (28 per
  * SM, 152 SMs): there the chain of one warp sets the time.  Four / two / one warps:
- * 2,048 particles 17 / 20 / 25 us, 32,768: 27 / 31 / 41 us, 131,946 (one fits): 86 / 66 / 59 us. */
+ * 2,048 particles 17 / 20 / 25 us, 32,768: 27 / 31 / 41 us, 131,946 (one fits): 86 / 66 / 59 us
+ * (blocks of four warps; one, now: 26 us at 32,768 with four, 48 at 131,946). */
 template<class R> void launch_nlist(const KArgs<R> &a, cudaStream_t st, int gated) {
     const int nw = a.npad / 32, room = 152 * 28;  // nw is a multiple of 8
     if (nw * 4 <= room)
