@@ -239,7 +239,7 @@ constexpr int SCAN_TILES = 4096;  // cell tiles per block of the tile scan
 
 // host-side launchers (explicitly instantiated for float and double)
 template<class R> void launch_rebuild(const KArgs<R> &a, cudaStream_t st, bool gated);
-// stage 0 rebin, 1 radix sort, 2 ranges + gather, 3 neighbour list
+// stage 0 rebin, 1 cell sort, 2 gather, 3 neighbour list
 template<class R> void launch_rebuild_stage(const KArgs<R> &a, cudaStream_t st, bool gated, int stage);
 template<class R> void launch_mesh(const KArgs<R> &a, cudaStream_t st);
 template<class R> void launch_step_langevin(const KArgs<R> &a, cudaStream_t st, bool energy);

@@ -1660,11 +1660,10 @@ template<class R> class Engine : public EngineBase {
             }
             return ORBC_OK;
         };
-        // the list-build form first (bits 3-4, at the caller's skin and the
-        // pipelined, inlined loop); then skin x force-loop form (bits 0-1, and
-        // the merged shell pass) with it; the skins half-way to the best one's
-        // grid neighbours; at the best pair the occupancy form (bit 2), the
-        // other list-build forms and two fixed rebuild cadences
+        // skin and cadence are what the trials decide; the form bits that they
+        // also vary (list build 3-4, force loop 0-1 and 5, occupancy 2) select the
+        // same kernels, and the table of trials keeps its rows for callers that
+        // read it
         const int occ0 = P.kernel_variant & 4, every0 = P.rebuild_every;
         const double skin0 = P.skin;
         for (int f = 0; f < 3; ++f)

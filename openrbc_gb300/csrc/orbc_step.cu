@@ -45,12 +45,10 @@ template<> __device__ __forceinline__ double4a ldg4<double>(const double4a *p) {
 }
 
 /* Streaming (evict-first) access for data touched once per step -- the
- * velocity / reference-position state and the neighbour rows of the plain
- * loops -- so that it does not push out of L2 the positions and orientations
- * that the next step gathers again.  The skin-shell rows, and the inner rows
- * of the merged loop, which every warp prefetches into L1 first, are read
- * through the read-only path instead (0.735 against 0.744 ms for the merged
- * form on the 4.03M cell). */
+ * velocity / reference-position state -- so that it does not push out of L2
+ * the positions and orientations that the next step gathers again.  The
+ * neighbour rows, which every warp prefetches into L1 first, are read through
+ * the read-only path. */
 template<class R> __device__ __forceinline__ typename Vec<R>::T4 ldcs4(const typename Vec<R>::T4 *p);
 template<> __device__ __forceinline__ float4 ldcs4<float>(const float4 *p) { return __ldcs(p); }
 template<> __device__ __forceinline__ double4a ldcs4<double>(const double4a *p) {
@@ -404,7 +402,14 @@ template<class R, bool EK, int U> constexpr int force_blocks() {
  * are the same for every U.  The hits that need the general pair table (a
  * protein partner, or an owner whose pairs with lipids are not anisotropic:
  * the list build puts all of these in the shell rows) follow.  All 32 lanes
- * of the warp must call it. */
+ * of the warp must call it.
+ *
+ * Bound by the L2 latency of the gathers (every row of a warp waits for its
+ * slowest lane) and, behind it, by issue (62 % of peak) and the L1 data pipe (67
+ * %).  On the 1.0M-particle cell a warp spends 9 of 42 thousand cycles on the
+ * shell rows, 23 on the others, 5 before and 5 after; the step kernel takes
+ * 0.174 ms (0.220 with votes on the pairs' types, range branches and the
+ * vertices' own walks; 122 against 166 million warp instructions). */
 template<class R, bool E, bool K, int U>
 __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, const OwnP<R> &P, R lim, int own_gen,
                                           int i, const typename Vec<R>::T4 *__restrict__ pos,
