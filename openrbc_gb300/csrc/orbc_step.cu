@@ -387,7 +387,7 @@ __device__ __forceinline__ void prefetch_warp_list(const uint32_t *nbr, int i, i
     }
 }
 
-/* Resident blocks of LITE_BS threads asked of the force kernels: FP32, 16 at
+/* Resident blocks asked of the force kernels: FP32, 16 at
  * 64 registers for batches of two rows (14 with energy or compensated sums,
  * which need more: EK), 10 for batches of four; the FP64 forms are bound by the FP64 pipe and
  * keep all the registers they need. */
@@ -941,10 +941,10 @@ __device__ __forceinline__ void langevin_particle(const KArgs<R> &a, const FFDev
  * the structure of the lite kernel below plus warp partials, summed per
  * system by k_reduce after the kernel. */
 template<class R, bool E, bool K, int U>
-__global__ void __launch_bounds__(LITE_BS, force_blocks<R, E || K, U>()) k_step_langevin(KArgs<R> a) {
+__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, E || K, U>()) k_step_langevin(KArgs<R> a) {
     using T4 = typename Vec<R>::T4;
-    __shared__ ShiftTab<R> shm[LITE_BS / 32];
-    const int i = blockIdx.x * LITE_BS + threadIdx.x;
+    __shared__ ShiftTab<R> shm[force_threads<R> / 32];
+    const int i = blockIdx.x * force_threads<R> + threadIdx.x;
     // the loads that depend on nothing, together
     const int4 sc = __ldcg(reinterpret_cast<const int4 *>(a.S));  // cur, lp, rebuild, error
     const int s = a.nsys > 1 ? a.blk_sys[i / SYS_PAD] : 0;
@@ -975,10 +975,10 @@ __global__ void __launch_bounds__(LITE_BS, force_blocks<R, E || K, U>()) k_step_
  * k_advance flips the buffers after the kernel.  The temperature is reduced on
  * demand (k_vcom). */
 template<class R, bool K, int U>
-__global__ void __launch_bounds__(LITE_BS, force_blocks<R, K, U>()) k_step_langevin_lite(KArgs<R> a) {
+__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, K, U>()) k_step_langevin_lite(KArgs<R> a) {
     using T4 = typename Vec<R>::T4;
-    __shared__ ShiftTab<R> shm[LITE_BS / 32];
-    const int i = blockIdx.x * LITE_BS + threadIdx.x;
+    __shared__ ShiftTab<R> shm[force_threads<R> / 32];
+    const int i = blockIdx.x * force_threads<R> + threadIdx.x;
     // the loads that depend on nothing, together
     const int4 sc = __ldcg(reinterpret_cast<const int4 *>(a.S));  // cur, lp, rebuild, error
     const int s = a.nsys > 1 ? a.blk_sys[i / SYS_PAD] : 0;
@@ -1031,11 +1031,11 @@ __global__ void k_advance(Scalars *S, int rebuild_every, int count_step, cudaGra
  * orientations ping-pong like the Langevin step; the step counter (the noise
  * key) does not advance. */
 template<class R, int U>
-__global__ void __launch_bounds__(LITE_BS, force_blocks<R, false, U>())
+__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, false, U>())
     k_minimize(KArgs<R> a, double dr_opt, double dn_opt) {
     using T4 = typename Vec<R>::T4;
-    __shared__ ShiftTab<R> shm[LITE_BS / 32];
-    const int i = blockIdx.x * LITE_BS + threadIdx.x;
+    __shared__ ShiftTab<R> shm[force_threads<R> / 32];
+    const int i = blockIdx.x * force_threads<R> + threadIdx.x;
     // the loads that depend on nothing, together
     const int4 sc = __ldcg(reinterpret_cast<const int4 *>(a.S));  // cur, lp, rebuild, error
     const int s = a.nsys > 1 ? a.blk_sys[i / SYS_PAD] : 0;
@@ -1098,10 +1098,10 @@ __global__ void __launch_bounds__(LITE_BS, force_blocks<R, false, U>())
  * fused with the forces: the lite structure plus warp partials for the
  * kinetic-energy sum that k_reduce turns into the thermostat update. */
 template<class R, bool E, bool K, int U>
-__global__ void __launch_bounds__(LITE_BS, force_blocks<R, E || K, U>()) k_nh_final(KArgs<R> a, int count_step) {
+__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, E || K, U>()) k_nh_final(KArgs<R> a, int count_step) {
     using T4 = typename Vec<R>::T4;
-    __shared__ ShiftTab<R> shm[LITE_BS / 32];
-    const int i = blockIdx.x * LITE_BS + threadIdx.x;
+    __shared__ ShiftTab<R> shm[force_threads<R> / 32];
+    const int i = blockIdx.x * force_threads<R> + threadIdx.x;
     // the loads that depend on nothing, together
     const int4 sc = __ldcg(reinterpret_cast<const int4 *>(a.S));  // cur, lp, rebuild, error
     const int s = a.nsys > 1 ? a.blk_sys[i / SYS_PAD] : 0;
@@ -1259,10 +1259,10 @@ template<class R> __global__ void __launch_bounds__(256) k_assign_temperature(KA
 }
 
 template<class R, bool K, int U>
-__global__ void __launch_bounds__(LITE_BS, force_blocks<R, true, U>()) k_forces(KArgs<R> a) {
+__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, true, U>()) k_forces(KArgs<R> a) {
     using T4 = typename Vec<R>::T4;
-    __shared__ ShiftTab<R> shm[LITE_BS / 32];
-    const int i = blockIdx.x * LITE_BS + threadIdx.x;
+    __shared__ ShiftTab<R> shm[force_threads<R> / 32];
+    const int i = blockIdx.x * force_threads<R> + threadIdx.x;
     // the loads that depend on nothing, together
     const int4 sc = __ldcg(reinterpret_cast<const int4 *>(a.S));  // cur, lp, rebuild, error
     const int s = a.nsys > 1 ? a.blk_sys[i / SYS_PAD] : 0;
@@ -1423,7 +1423,7 @@ template<class R> void reduce_sums(const KArgs<R> &a, int mode, int count_step, 
  * 29 / 34 us, 1.0M: 174 / 243 us.  FP64: one row (the FP64 pipe is the bound:
  * 1.11 against 1.13 and 1.15 ms on a 250 thousand particle cell). */
 template<class R, class L> void by_batch(const KArgs<R> &a, L launch) {
-    const int nb = a.npad / LITE_BS;
+    const int nb = a.npad / force_threads<R>;
     if constexpr (sizeof(R) == 8)
         launch(std::integral_constant<int, 1>(), nb);
     else if (nb <= 152 * force_blocks<R, false, 4>())
@@ -1435,11 +1435,11 @@ template<class R, bool K> void step_langevin_v(const KArgs<R> &a, cudaStream_t s
     by_batch<R>(a, [&](auto u, int nb) {
         constexpr int U = decltype(u)::value;
         if (energy)
-            k_step_langevin<R, true, K, U><<<nb, LITE_BS, 0, st>>>(a);
+            k_step_langevin<R, true, K, U><<<nb, force_threads<R>, 0, st>>>(a);
         else if (a.zero_bulk)
-            k_step_langevin<R, false, K, U><<<nb, LITE_BS, 0, st>>>(a);
+            k_step_langevin<R, false, K, U><<<nb, force_threads<R>, 0, st>>>(a);
         else
-            k_step_langevin_lite<R, K, U><<<nb, LITE_BS, 0, st>>>(a);
+            k_step_langevin_lite<R, K, U><<<nb, force_threads<R>, 0, st>>>(a);
     });
     if (energy || a.zero_bulk)
         reduce_sums<R>(a, MODE_LANGEVIN, 1, st);
@@ -1456,9 +1456,9 @@ template<class R, bool K> void nh_final_v(const KArgs<R> &a, cudaStream_t st, bo
     by_batch<R>(a, [&](auto u, int nb) {
         constexpr int U = decltype(u)::value;
         if (energy)
-            k_nh_final<R, true, K, U><<<nb, LITE_BS, 0, st>>>(a, count_step);
+            k_nh_final<R, true, K, U><<<nb, force_threads<R>, 0, st>>>(a, count_step);
         else
-            k_nh_final<R, false, K, U><<<nb, LITE_BS, 0, st>>>(a, count_step);
+            k_nh_final<R, false, K, U><<<nb, force_threads<R>, 0, st>>>(a, count_step);
     });
     reduce_sums<R>(a, MODE_NH_FINAL, count_step, st);
 }
@@ -1482,9 +1482,9 @@ template<class R> void launch_forces(const KArgs<R> &a, cudaStream_t st) {
     by_batch<R>(a, [&](auto u, int nb) {
         constexpr int U = decltype(u)::value;
         if (a.kahan)
-            k_forces<R, true, U><<<nb, LITE_BS, 0, st>>>(a);
+            k_forces<R, true, U><<<nb, force_threads<R>, 0, st>>>(a);
         else
-            k_forces<R, false, U><<<nb, LITE_BS, 0, st>>>(a);
+            k_forces<R, false, U><<<nb, force_threads<R>, 0, st>>>(a);
     });
     reduce_sums<R>(a, MODE_FORCES, 0, st);
 }
@@ -1493,7 +1493,7 @@ template<class R> void launch_mesh(const KArgs<R> &a, cudaStream_t st) {
 }
 template<class R> void launch_minimize(const KArgs<R> &a, double dr_opt, double dn_opt, cudaStream_t st) {
     by_batch<R>(a, [&](auto u, int nb) {
-        k_minimize<R, decltype(u)::value><<<nb, LITE_BS, 0, st>>>(a, dr_opt, dn_opt);
+        k_minimize<R, decltype(u)::value><<<nb, force_threads<R>, 0, st>>>(a, dr_opt, dn_opt);
     });
     k_advance<<<1, 1, 0, st>>>(a.S, a.rebuild_every, 0, a.cond, a.has_cond);
 }
