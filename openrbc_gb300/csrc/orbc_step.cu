@@ -309,8 +309,10 @@ __device__ __forceinline__ double positive_part(double x) { return __double2hiin
  *   f = sum (cu d + kj n_j) + n_i sum kd,   t = sum (kd d - au n_j)
  * with d = x_i - x_j, niu = n_i.d / r, nju = n_j.d / r and the coefficients of
  * src/pairwise_kernel.h:30-68.  Pairs outside the range enter with r_c - r
- * clamped to 0, so that every coefficient vanishes and no branch is needed.
- * Each operation is rounded as written, so the sums do not depend on how the
+ * clamped to 0, so that every coefficient vanishes and no branch is needed; a
+ * normal that is not a number would still get through (0 x NaN), so IN_RANGE
+ * leaves such pairs out by a branch, for the rare warp that meets one.  Each
+ * operation is rounded as written, so the sums do not depend on how the
  * loops around them are compiled. */
 template<class R> struct OwnP {
     R cut, rep8, a0, a1, aatt, hrep;  // a0 = 4 att (1 - alpha), a1 = 4 att alpha, hrep = rep / 2
@@ -337,7 +339,7 @@ template<class R, bool K> struct PairAcc {
         e = R(0);
     }
 };
-template<class R, bool E, bool K>
+template<class R, bool E, bool K, bool IN_RANGE>
 __device__ __forceinline__ void pair_term(PairAcc<R, K> &A, const OwnP<R> &P, const R d[3], const R n[3], R nix, R niy,
                                           R niz) {
     const R r2 = fma_rn(d[2], d[2], fma_rn(d[1], d[1], mul_rn(d[0], d[0])));
@@ -354,6 +356,7 @@ __device__ __forceinline__ void pair_term(PairAcc<R, K> &A, const OwnP<R> &P, co
     const R auar = mul_rn(au, ri);
     const R kd = mul_rn(auar, nju), kj = mul_rn(auar, niu);
     const R cu = mul_rn(fma_rn(kd, mul_rn(niu, R(-2)), fra), ri);
+    if (IN_RANGE && !(rc > R(0))) return;
     if (K) {
 #pragma unroll
         for (int k = 0; k < NACC; ++k) {
@@ -410,7 +413,7 @@ template<class R, bool EK, int U> constexpr int force_blocks() {
  * shell rows, 23 on the others, 5 before and 5 after; the step kernel takes
  * 0.174 ms (0.220 with votes on the pairs' types, range branches and the
  * vertices' own walks; 122 against 166 million warp instructions). */
-template<class R, bool E, bool K, int U>
+template<class R, bool E, bool K, int U, bool IN_RANGE>
 __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, const OwnP<R> &P, R lim, int own_gen,
                                           int i, const typename Vec<R>::T4 *__restrict__ pos,
                                           const typename Vec<R>::T4 *__restrict__ nrm, int ty, int packed,
@@ -433,7 +436,7 @@ __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, 
         R d[3];
         const R n[3] = {nj.x, nj.y, nj.z};
         offset(ent, pj, d);
-        pair_term<R, E, K>(A, P, d, n, ni.x, ni.y, ni.z);
+        pair_term<R, E, K, IN_RANGE>(A, P, d, n, ni.x, ni.y, ni.z);
     };
     // rows that every lane still has inside (rounded down to whole batches): no selection
     int kmin = int(__reduce_min_sync(0xffffffffu, unsigned(nin))) / U * U;
@@ -500,7 +503,7 @@ __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, 
                         R d[3];
                         const R n[3] = {nj[u].x, nj[u].y, nj[u].z};
                         offset(ent[u], pj[u], d);
-                        pair_term<R, E, K>(A, own_params(q), d, n, ni.x, ni.y, ni.z);
+                        pair_term<R, E, K, IN_RANGE>(A, own_params(q), d, n, ni.x, ni.y, ni.z);
                     } else {
                         hb |= bit[u];
                     }
@@ -640,6 +643,7 @@ __device__ __forceinline__ void slot_forces(const KArgs<R> &a, const FFDev<R> &F
                                             const typename Vec<R>::T4 &pi, const typename Vec<R>::T4 &ni,
                                             const SysDev &sd, const SysState &ss, int packed,
                                             const ShiftTab<R> &sh, R3<R> &f, R3<R> &t, R &e, int &flags) {
+    using T4 = typename Vec<R>::T4;
     const bool real = w_type(w) != GHOST;
     const int ty = real ? w_type(w) : 0;
     const PairP<R> &pl = F.pair[ty * NT];  // with a lipid
@@ -648,14 +652,29 @@ __device__ __forceinline__ void slot_forces(const KArgs<R> &a, const FFDev<R> &F
     A.clear();
     const R lim = F.reach2[ty];
     const int own_gen = pl.kind == PAIR_ANISO ? 0 : 1;
-    pair_sums<R, E, K, U>(a, F, P, lim, own_gen, i, a.pos[cur], a.nrm[cur], ty, packed, pi, ni, sh, A);
+    T4 na = ni;  // not used by a type without anisotropic pairs, which may carry anything there
+    if (own_gen) na.x = na.y = na.z = R(0);
+    const T4 *__restrict__ pos = a.pos[cur], *__restrict__ nrm = a.nrm[cur];
+    pair_sums<R, E, K, U, false>(a, F, P, lim, own_gen, i, pos, nrm, ty, packed, pi, na, sh, A);
+    const R sum = add_rn(add_rn(add_rn(A.s[0], A.s[1]), add_rn(A.s[2], A.s[3])),
+                         add_rn(add_rn(A.s[4], A.s[5]), A.s[6]));
+    if (__any_sync(0xffffffffu, sum != sum)) {
+        // again with the pairs in range alone.  What the sums take is read anew: kept in registers until here,
+        // it would cost the common path spills
+        asm volatile("" ::: "memory");
+        const PairP<R> &pl2 = F.pair[ty * NT];
+        A.clear();
+        pair_sums<R, E, K, 1, true>(a, F, own_params(pl2), F.reach2[ty], pl2.kind == PAIR_ANISO ? 0 : 1, i, pos, nrm,
+                                    ty, __ldcg(a.nnb + i), pi, na, sh, A);
+    }
+    if (A.s[6] == R(0)) na.x = na.y = na.z = R(0);
     if (K) {
 #pragma unroll
         for (int k = 0; k < NACC; ++k) A.s[k] = add_rn(A.s[k], -A.c[K ? k : 0]);
     }
-    f.x = fma_rn(A.s[6], ni.x, A.s[0]);
-    f.y = fma_rn(A.s[6], ni.y, A.s[1]);
-    f.z = fma_rn(A.s[6], ni.z, A.s[2]);
+    f.x = fma_rn(A.s[6], na.x, A.s[0]);
+    f.y = fma_rn(A.s[6], na.y, A.s[1]);
+    f.z = fma_rn(A.s[6], na.z, A.s[2]);
     t.x = A.s[3];
     t.y = A.s[4];
     t.z = A.s[5];
