@@ -390,32 +390,36 @@ __device__ __forceinline__ void prefetch_warp_list(const uint32_t *nbr, int i, i
     }
 }
 
-/* Resident blocks asked of the force kernels: FP32, 16 at
- * 64 registers for batches of two rows (14 with energy or compensated sums,
- * which need more: EK), 10 for batches of four; the FP64 forms are bound by the FP64 pipe and
- * keep all the registers they need. */
-template<class R, bool EK, int U> constexpr int force_blocks() {
-    return sizeof(R) == 8 ? 1 : U == 2 ? (EK ? 14 : 16) : 10;
+/* Resident blocks asked of the force kernels: FP32, 16 at 64 registers for
+ * batches of two rows (14 at 72 with compensated sums, which need more), 10
+ * for batches of four; the FP64 forms are bound by the FP64 pipe and keep all
+ * the registers they need (16 blocks and more: 840 -> 850 us on a 250 thousand
+ * particle cell). */
+template<class R, bool K, int U> constexpr int force_blocks() {
+    return sizeof(R) == 8 ? 1 : U == 2 ? (K ? 14 : 16) : 10;
 }
 
 /* Pair sums of slot i over its list.  Shell rows are tested first, 32 at a
- * time; a hit is a bit of a mask.  Then the inner rows and the lipids among
- * the hits go through one loop, U of them at a time: their entries and
- * gathers are issued together and their terms added in row order, so the sums
- * are the same for every U.  The hits that need the general pair table (a
- * protein partner, or an owner whose pairs with lipids are not anisotropic:
- * the list build puts all of these in the shell rows) follow.  All 32 lanes
- * of the warp must call it.
+ * time; a hit is a bit of a mask.  Then the inner rows and the hits go through
+ * one loop, U of them at a time: their entries and gathers are issued together
+ * and their terms added in row order, so the sums are the same for every U.  A
+ * lipid's hits among the proteins that it has anisotropic pairs with take the
+ * same arithmetic with their own parameters; the hits that need the general
+ * pair table (two proteins, or a type without anisotropic pairs: the list
+ * build puts all of these in the shell rows) follow if they are in range.  All
+ * 32 lanes of the warp must call it.
  *
  * Bound by the L2 latency of the gathers (every row of a warp waits for its
- * slowest lane) and, behind it, by issue (62 % of peak) and the L1 data pipe (67
- * %).  On the 1.0M-particle cell a warp spends 9 of 42 thousand cycles on the
- * shell rows, 23 on the others, 5 before and 5 after; the step kernel takes
- * 0.174 ms (0.220 with votes on the pairs' types, range branches and the
- * vertices' own walks; 122 against 166 million warp instructions). */
+ * slowest lane) and, behind it, by issue and the L1 data pipe.  On the
+ * 1.0M-particle cell a warp spends 9 of 42 thousand cycles on the shell rows, 23
+ * on the others, 5 before and 5 after.  A cell with 17 % proteins (0.91M
+ * particles) has a lane without anisotropic pairs in almost every warp: 160 us
+ * per step kernel against 183 with such lanes left out of the loop without
+ * selection, their general hits walked unconditionally and the lipids'
+ * protein pairs in a branch of their own; FP64, 0.23M particles, 860 -> 740. */
 template<class R, bool E, bool K, int U, bool IN_RANGE>
-__device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, const OwnP<R> &P, R lim, int own_gen,
-                                          int i, const typename Vec<R>::T4 *__restrict__ pos,
+__device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, const OwnP<R> &P, int i,
+                                          const typename Vec<R>::T4 *__restrict__ pos,
                                           const typename Vec<R>::T4 *__restrict__ nrm, int ty, int packed,
                                           const typename Vec<R>::T4 &pi, const typename Vec<R>::T4 &ni,
                                           const ShiftTab<R> &sh, PairAcc<R, K> &A) {
@@ -438,10 +442,9 @@ __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, 
         offset(ent, pj, d);
         pair_term<R, E, K, IN_RANGE>(A, P, d, n, ni.x, ni.y, ni.z);
     };
-    // rows that every lane still has inside (rounded down to whole batches): no selection
-    int kmin = int(__reduce_min_sync(0xffffffffu, unsigned(nin))) / U * U;
     for (int k0 = 0;; k0 += 32) {
-        uint32_t hm = 0u, hb = 0u;
+        uint32_t hm = 0u, hb = 0u;  // hits: for the rows' loop, for the general table
+        const R lim = F.reach2[ty];
         const int nq = min(32, nout - k0);
         const int nqmax = int(__reduce_max_sync(0xffffffffu, unsigned(max(nq, 0))));
         for (int k = 0; k < nqmax; k += SHELL_U) {
@@ -455,7 +458,15 @@ __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, 
             for (int u = 0; u < SHELL_U; ++u) {
                 if constexpr (sizeof(R) == 8) {
                     const bool in = shell_inside(sh, pi, pj[u], int(ent[u] >> NB_SHIFT), lim);
-                    if (k + u < nq && in) hm |= 1u << (k + u);
+                    if (k + u < nq && in) {
+                        // the general pairs are told apart here, each by its own range: a row of the loop
+                        // below costs the FP64 pipe 60 operations
+                        const PairP<R> &q = F.pair[ty * NT + w_type(wbits(pj[u].w))];
+                        if (q.kind == PAIR_ANISO)
+                            hm |= 1u << (k + u);
+                        else if (shell_inside(sh, pi, pj[u], int(ent[u] >> NB_SHIFT), q.anysq))
+                            hb |= 1u << (k + u);
+                    }
                 } else {
                     R d[3];
                     offset(ent[u], pj[u], d);
@@ -463,7 +474,19 @@ __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, 
                 }
             }
         }
-        const int total = int(__reduce_max_sync(0xffffffffu, unsigned(nin + __popc(hm))));
+        // rows that every lane still has inside (rounded down to whole batches): no selection.  A lane without
+        // anisotropic pairs has no rows, and goes along on those of a lane that has: its own parameters make
+        // them vanish
+        const unsigned with = k0 == 0 ? __ballot_sync(0xffffffffu, P.cut > R(0)) : 0u;
+        int kmin = 0;
+        if (with) {
+            kmin = int(__reduce_min_sync(0xffffffffu, unsigned(P.cut > R(0) ? nin : 0xffff))) / U * U;
+            if (!(P.cut > R(0))) {
+                nin = kmin;
+                nb += __ffs(int(with)) - 1 - int(threadIdx.x & 31);
+            }
+        }
+#pragma unroll 1
         for (int k = 0; k < kmin; k += U) {
             uint32_t ent[U];
             T4 pj[U], nj[U];
@@ -477,6 +500,8 @@ __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, 
 #pragma unroll
             for (int u = 0; u < U; ++u) term(ent[u], pj[u], nj[u]);
         }
+        nb = a.nbr + nbr_index(i, 0, a.cap);
+        const int total = int(__reduce_max_sync(0xffffffffu, unsigned(nin + __popc(hm))));
         for (int k = kmin; k < total; k += U) {
             uint32_t ent[U], bit[U];
             T4 pj[U], nj[U];
@@ -496,20 +521,21 @@ __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, 
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int tj = w_type(wbits(pj[u].w));
-                if (bit[u] && (tj | own_gen) != 0) {
+                OwnP<R> Q = P;
+                R d[3], n[3] = {nj[u].x, nj[u].y, nj[u].z};
+                offset(ent[u], pj[u], d);
+                if (bit[u] && (tj != 0 || !(P.cut > R(0)))) {
                     // a lipid's pair with a protein has parameters of its own; the rest waits
                     const PairP<R> &q = F.pair[ty * NT + tj];
                     if (ty == 0 && q.kind == PAIR_ANISO) {
-                        R d[3];
-                        const R n[3] = {nj[u].x, nj[u].y, nj[u].z};
-                        offset(ent[u], pj[u], d);
-                        pair_term<R, E, K, IN_RANGE>(A, own_params(q), d, n, ni.x, ni.y, ni.z);
+                        Q = own_params(q);
                     } else {
-                        hb |= bit[u];
+                        Q.cut = R(0);
+                        n[0] = n[1] = n[2] = R(0);
+                        if (dist2(d) < q.anysq) hb |= bit[u];
                     }
-                } else {
-                    term(ent[u], pj[u], nj[u]);
                 }
+                pair_term<R, E, K, IN_RANGE>(A, Q, d, n, ni.x, ni.y, ni.z);
             }
         }
         // the general pairs among the hits
@@ -534,7 +560,7 @@ __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, 
             if (E) A.e = add_rn(A.e, ee);
         }
         if (!__any_sync(0xffffffffu, nout > k0 + 32)) break;
-        nin = kmin = 0;
+        nin = 0;
     }
 }
 
@@ -650,12 +676,10 @@ __device__ __forceinline__ void slot_forces(const KArgs<R> &a, const FFDev<R> &F
     const OwnP<R> P = own_params(pl);
     PairAcc<R, K> A;
     A.clear();
-    const R lim = F.reach2[ty];
-    const int own_gen = pl.kind == PAIR_ANISO ? 0 : 1;
     T4 na = ni;  // not used by a type without anisotropic pairs, which may carry anything there
-    if (own_gen) na.x = na.y = na.z = R(0);
+    if (!(P.cut > R(0))) na.x = na.y = na.z = R(0);
     const T4 *__restrict__ pos = a.pos[cur], *__restrict__ nrm = a.nrm[cur];
-    pair_sums<R, E, K, U, false>(a, F, P, lim, own_gen, i, pos, nrm, ty, packed, pi, na, sh, A);
+    pair_sums<R, E, K, U, false>(a, F, P, i, pos, nrm, ty, packed, pi, na, sh, A);
     const R sum = add_rn(add_rn(add_rn(A.s[0], A.s[1]), add_rn(A.s[2], A.s[3])),
                          add_rn(add_rn(A.s[4], A.s[5]), A.s[6]));
     if (__any_sync(0xffffffffu, sum != sum)) {
@@ -664,8 +688,7 @@ __device__ __forceinline__ void slot_forces(const KArgs<R> &a, const FFDev<R> &F
         asm volatile("" ::: "memory");
         const PairP<R> &pl2 = F.pair[ty * NT];
         A.clear();
-        pair_sums<R, E, K, 1, true>(a, F, own_params(pl2), F.reach2[ty], pl2.kind == PAIR_ANISO ? 0 : 1, i, pos, nrm,
-                                    ty, __ldcg(a.nnb + i), pi, na, sh, A);
+        pair_sums<R, E, K, 1, true>(a, F, own_params(pl2), i, pos, nrm, ty, __ldcg(a.nnb + i), pi, na, sh, A);
     }
     if (A.s[6] == R(0)) na.x = na.y = na.z = R(0);
     if (K) {
@@ -960,7 +983,7 @@ __device__ __forceinline__ void langevin_particle(const KArgs<R> &a, const FFDev
  * the structure of the lite kernel below plus warp partials, summed per
  * system by k_reduce after the kernel. */
 template<class R, bool E, bool K, int U>
-__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, E || K, U>()) k_step_langevin(KArgs<R> a) {
+__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, K, U>()) k_step_langevin(KArgs<R> a) {
     using T4 = typename Vec<R>::T4;
     __shared__ ShiftTab<R> shm[force_threads<R> / 32];
     const int i = blockIdx.x * force_threads<R> + threadIdx.x;
@@ -1117,7 +1140,7 @@ __global__ void __launch_bounds__(force_threads<R>, force_blocks<R, false, U>())
  * fused with the forces: the lite structure plus warp partials for the
  * kinetic-energy sum that k_reduce turns into the thermostat update. */
 template<class R, bool E, bool K, int U>
-__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, E || K, U>()) k_nh_final(KArgs<R> a, int count_step) {
+__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, K, U>()) k_nh_final(KArgs<R> a, int count_step) {
     using T4 = typename Vec<R>::T4;
     __shared__ ShiftTab<R> shm[force_threads<R> / 32];
     const int i = blockIdx.x * force_threads<R> + threadIdx.x;
@@ -1278,7 +1301,7 @@ template<class R> __global__ void __launch_bounds__(256) k_assign_temperature(KA
 }
 
 template<class R, bool K, int U>
-__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, true, U>()) k_forces(KArgs<R> a) {
+__global__ void __launch_bounds__(force_threads<R>, force_blocks<R, K, U>()) k_forces(KArgs<R> a) {
     using T4 = typename Vec<R>::T4;
     __shared__ ShiftTab<R> shm[force_threads<R> / 32];
     const int i = blockIdx.x * force_threads<R> + threadIdx.x;
