@@ -791,7 +791,13 @@ __device__ __forceinline__ void warp_partials(const KArgs<R> &a, int i, R ke, R 
     }
 }
 
-__device__ __forceinline__ double max_or_nan(double x, double y) { return (x > y || !(x == x)) ? x : y; }
+/* The larger of two numbers >= 0, or the one that is not a number, by their
+ * bits: two FP64 comparisons per step of the tree instead cost k_reduce 2 us of
+ * 20 (908 thousand particles). */
+__device__ __forceinline__ double max_or_nan(double x, double y) {
+    const unsigned long long a = __double_as_longlong(x), b = __double_as_longlong(y);
+    return __longlong_as_double((long long)(a > b ? a : b));
+}
 __device__ __forceinline__ double combine_part(int k, double x, double y) {
     return k == 2 ? max_or_nan(x, y) : (k == 3 ? double(int(x) | int(y)) : x + y);
 }
