@@ -17,6 +17,7 @@
 //                    around its own; the last block flips buffer parities
 #include "orbc_device.cuh"
 
+#include <algorithm>
 #include <cstdio>
 #include <type_traits>
 
@@ -244,8 +245,12 @@ template<class R> __global__ void __launch_bounds__(256) k_rebin(KArgs<R> a, int
     }
 }
 
+constexpr int SCAN_GRID = 152 * 2;  // resident blocks of the tile scan
 /* Exclusive prefix of the tiles' particle counts inside each block of
- * SCAN_TILES; the last block to finish turns the block totals into prefixes. */
+ * SCAN_TILES; the last block to finish turns the block totals into prefixes.
+ * The grid is bounded (SCAN_GRID), as an open system with a stray particle may have
+ * 10^9 cells, almost all of them empty: 1.7e9 cells, 2,000 particles, rebuild 187 ->
+ * 102 us, and the launches of a chain that finds the gate closed 230 -> 44. */
 __global__ void __launch_bounds__(1024) k_tile_scan(const int *tcnt, int *tstart, int *bsum, int nscan,
                                                     unsigned int *counter, const int *gate) {
     if (gate_closed(gate)) return;
@@ -274,13 +279,24 @@ __global__ void __launch_bounds__(1024) k_tile_scan(const int *tcnt, int *tstart
         __syncthreads();
         return x + (warp > 0 ? wsum[warp - 1] : 0);
     };
-    const int64_t q = int64_t(blockIdx.x) * (SCAN_TILES / 4) + t;
-    const int4 c = reinterpret_cast<const int4 *>(tcnt)[q];
-    const int sum = c.x + c.y + c.z + c.w;
-    const int e = scan(sum) - sum;
-    reinterpret_cast<int4 *>(tstart)[q] = make_int4(e, e + c.x, e + c.x + c.y, e + c.x + c.y + c.z);
+    auto load = [&](int b) {
+        return b < nscan ? reinterpret_cast<const int4 *>(tcnt)[int64_t(b) * (SCAN_TILES / 4) + t] : make_int4(0, 0, 0, 0);
+    };
+    int4 c = load(blockIdx.x);
+    for (int b = blockIdx.x; b < nscan; b += gridDim.x) {
+        const int4 next = load(b + gridDim.x);
+        const int sum = c.x + c.y + c.z + c.w;
+        int total = 0;
+        if (__syncthreads_or(sum)) {  // the prefixes of empty tiles are not read
+            const int e = scan(sum) - sum;
+            reinterpret_cast<int4 *>(tstart)[int64_t(b) * (SCAN_TILES / 4) + t] =
+                make_int4(e, e + c.x, e + c.x + c.y, e + c.x + c.y + c.z);
+            total = wsum[31];
+        }
+        if (t == 0) bsum[b] = total;
+        c = next;
+    }
     if (t == 0) {
-        bsum[blockIdx.x] = wsum[31];
         __threadfence();
         last = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
@@ -303,40 +319,45 @@ __global__ void __launch_bounds__(1024) k_tile_scan(const int *tcnt, int *tstart
 template<class R> __global__ void __launch_bounds__(256) k_tile_cells(KArgs<R> a, int gated) {
     if (gated && !__ldcg(&a.S->rebuild)) return;
     const int lane = threadIdx.x & 31;
-    const int t0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 32;
-    if (t0 >= a.nctile) return;
     if (blockIdx.x == 0)
         for (int s = threadIdx.x; s < a.nsys; s += blockDim.x) a.gcnt[s] = 0;
-    const int n = a.tcnt[t0 + lane];  // nctile is a multiple of 32
-    const int start = n ? a.tstart[t0 + lane] + a.bsum[(t0 + lane) / SCAN_TILES] : 0;
-    if (n) a.tcnt[t0 + lane] = 0;
-    for (unsigned m = __ballot_sync(0xffffffffu, n != 0); m; m &= m - 1u) {
-        const int l = __ffs(int(m)) - 1;
-        const int64_t id0 = int64_t(t0 + l) * 64;
-        int lo = 0, hi = a.nsys - 1;  // the system whose ids these are
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) / 2;
-            if (int64_t(a.sys[mid].cell_base) <= id0)
-                lo = mid;
-            else
-                hi = mid - 1;
+    const int stride = int(gridDim.x) * 256;
+    for (int t0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; t0 < a.nctile; t0 += stride) {
+        if (stride < a.nctile) {  // scan blocks without particles are passed over
+            const int b = t0 / SCAN_TILES;
+            if (b + 1 < a.nscan && a.bsum[b] == a.bsum[b + 1]) continue;
         }
-        const int base = __shfl_sync(0xffffffffu, start, l) + a.sys[lo].slot_shift;
-        const int c0 = a.ccnt[id0 + 2 * lane], c1 = a.ccnt[id0 + 2 * lane + 1];
-        int x = c0 + c1;
+        const int n = a.tcnt[t0 + lane];  // nctile is a multiple of 32
+        const int start = n ? a.tstart[t0 + lane] + a.bsum[(t0 + lane) / SCAN_TILES] : 0;
+        if (n) a.tcnt[t0 + lane] = 0;
+        for (unsigned m = __ballot_sync(0xffffffffu, n != 0); m; m &= m - 1u) {
+            const int l = __ffs(int(m)) - 1;
+            const int64_t id0 = int64_t(t0 + l) * 64;
+            int lo = 0, hi = a.nsys - 1;  // the system whose ids these are
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) / 2;
+                if (int64_t(a.sys[mid].cell_base) <= id0)
+                    lo = mid;
+                else
+                    hi = mid - 1;
+            }
+            const int base = __shfl_sync(0xffffffffu, start, l) + a.sys[lo].slot_shift;
+            const int c0 = a.ccnt[id0 + 2 * lane], c1 = a.ccnt[id0 + 2 * lane + 1];
+            int x = c0 + c1;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        const int b = base + x - c0 - c1;
-        if (c0) {
-            a.ranges[id0 + 2 * lane] = make_int2(b, b + c0);
-            a.ccnt[id0 + 2 * lane] = 0;
-        }
-        if (c1) {
-            a.ranges[id0 + 2 * lane + 1] = make_int2(b + c0, b + c0 + c1);
-            a.ccnt[id0 + 2 * lane + 1] = 0;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            const int b = base + x - c0 - c1;
+            if (c0) {
+                a.ranges[id0 + 2 * lane] = make_int2(b, b + c0);
+                a.ccnt[id0 + 2 * lane] = 0;
+            }
+            if (c1) {
+                a.ranges[id0 + 2 * lane + 1] = make_int2(b + c0, b + c0 + c1);
+                a.ccnt[id0 + 2 * lane + 1] = 0;
+            }
         }
     }
 }
@@ -816,9 +837,10 @@ template<class R> void launch_rebuild_stage(const KArgs<R> &a, cudaStream_t st, 
             k_rebin<R><<<a.npad / 256, 256, 0, st>>>(a, gated ? 1 : 0);
             break;
         case 1:
-            k_tile_scan<<<a.nscan, 1024, 0, st>>>(a.tcnt, a.tstart, a.bsum, a.nscan, &a.S->scan_counter,
-                                                  gated ? &a.S->rebuild : nullptr);
-            k_tile_cells<R><<<a.nctile / 256, 256, 0, st>>>(a, gated ? 1 : 0);
+            k_tile_scan<<<std::min(a.nscan, SCAN_GRID), 1024, 0, st>>>(a.tcnt, a.tstart, a.bsum, a.nscan,
+                                                                       &a.S->scan_counter,
+                                                                       gated ? &a.S->rebuild : nullptr);
+            k_tile_cells<R><<<std::min(a.nctile / 256, 16 * SCAN_GRID), 256, 0, st>>>(a, gated ? 1 : 0);
             k_place<R><<<a.npad / 256, 256, 0, st>>>(a, gated ? 1 : 0);
             k_rank<R><<<a.npad / 256, 256, 0, st>>>(a, gated ? 1 : 0);
             break;
