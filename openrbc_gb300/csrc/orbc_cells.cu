@@ -245,7 +245,7 @@ template<class R> __global__ void __launch_bounds__(256) k_rebin(KArgs<R> a, int
     }
 }
 
-constexpr int SCAN_GRID = 152 * 2;  // resident blocks of the tile scan
+constexpr int SCAN_GRID = NUM_SM * 2;  // resident blocks of the tile scan
 /* Exclusive prefix of the tiles' particle counts inside each block of
  * SCAN_TILES; the last block to finish turns the block totals into prefixes.
  * The grid is bounded (SCAN_GRID), as an open system with a stray particle may have
@@ -498,7 +498,8 @@ template<class R> __device__ __forceinline__ void nlist_finalise(const KArgs<R> 
 // fewer passes per warp.  Blocks of two warps: one of four holds its memory until
 // its slowest warp is done (4.03M 1.08 ms), single warps fit only 26 (1.10 ms).
 constexpr int NLW = 2;  // warps per block of the list build
-template<class R, int SW> __global__ void __launch_bounds__(32 * NLW, (sizeof(R) == 8 ? 24 : 28) / NLW) k_nlist(KArgs<R> a, int gated) {
+template<class R> constexpr int nlist_warps = sizeof(R) == 8 ? 24 : 28;  // resident per SM
+template<class R, int SW> __global__ void __launch_bounds__(32 * NLW, nlist_warps<R> / NLW) k_nlist(KArgs<R> a, int gated) {
     using T4 = typename Vec<R>::T4;
     if (gated && !__ldcg(&a.S->rebuild)) return;
     constexpr int MB = 8;                                 // accept masks (32 candidates each) per lane
@@ -810,12 +811,14 @@ template<class R, int SW> __global__ void __launch_bounds__(32 * NLW, (sizeof(R)
     nlist_finalise(a, real ? qtot : 0, cur, lp);
 }
 
-/* As many warps per 32 slots (4, 2 or 1) as are all resident at once (28 per
- * SM, 152 SMs): there the chain of one warp sets the time.  Four / two / one warps:
- * 2,048 particles 17 / 20 / 25 us, 32,768: 27 / 31 / 41 us, 131,946 (one fits): 86 / 66 / 59 us
- * (blocks of four warps; one, now: 26 us at 32,768 with four, 48 at 131,946). */
+/* As many warps per 32 slots (4, 2 or 1) as are all resident at once: there the
+ * chain of one warp sets the time.  Four / two / one warps, FP32 (4,256 resident):
+ * 2,048 particles 16 / 17 / 22 us, 34,000 (four fit) 22 / 22 / 25, 40,000 33 / 22 / 25, 67,000
+ * (two fit) 42 / 27 / 28, 75,000 47 / 38 / 29, 200,000 115 / 75 / 59; FP64 (3,648): 2,048 21 / 29 /
+ * 43 us, 26,000 (four fit) 33 / 33 / 45, 32,768 47 / 36 / 45, 58,000 (two fit) 65 / 52 / 52, 62,000 73 /
+ * 69 / 55. */
 template<class R> void launch_nlist(const KArgs<R> &a, cudaStream_t st, int gated) {
-    const int nw = a.npad / 32, room = 152 * 28;  // nw is a multiple of 8
+    const int nw = a.npad / 32, room = NUM_SM * nlist_warps<R>;  // nw is a multiple of 8
     if (nw * 4 <= room)
         k_nlist<R, 4><<<nw * 4 / NLW, 32 * NLW, 0, st>>>(a, gated);
     else if (nw * 2 <= room)
@@ -826,7 +829,7 @@ template<class R> void launch_nlist(const KArgs<R> &a, cudaStream_t st, int gate
 
 static int grid_for(int64_t n, int per_block = 256) {
     int64_t g = (n + per_block - 1) / per_block;
-    const int64_t cap = 152 * 8;
+    const int64_t cap = NUM_SM * 8;
     return int(g < 1 ? 1 : (g > cap ? cap : g));
 }
 

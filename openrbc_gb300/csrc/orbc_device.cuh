@@ -21,6 +21,7 @@ namespace orbc {
 constexpr int NT = 6;            // particle types (src/forcefield_canonical.h:31-37)
 constexpr int GHOST = 15;        // type of padding slots
 constexpr int SYS_PAD = 256;     // slot padding per system
+constexpr int NUM_SM = 152;      // SMs of a GB300: the rules that ask whether a grid is resident at once
 // threads per block of the force / integrator kernels: two warps, which share their gathers in L1; one in
 // FP64, where nothing waits on L1 and a block should not hold its registers for its slower warp (32,768
 // lattice: step kernel 99 -> 90 us; in FP32 the 1.0M cell goes from 0.174 to 0.190 ms)

@@ -1474,7 +1474,7 @@ template<class R, class L> void by_batch(const KArgs<R> &a, L launch) {
     const int nb = a.npad / force_threads<R>;
     if constexpr (sizeof(R) == 8)
         launch(std::integral_constant<int, 1>(), nb);
-    else if (nb <= 152 * force_blocks<R, false, 4>())
+    else if (nb <= NUM_SM * force_blocks<R, false, 4>())
         launch(std::integral_constant<int, 4>(), nb);
     else
         launch(std::integral_constant<int, 2>(), nb);
