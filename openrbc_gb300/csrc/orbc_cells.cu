@@ -538,11 +538,10 @@ template<class R, int SW> __global__ void __launch_bounds__(32 * NLW, nlist_warp
         const R ex = pi.x - qs.x, ey = pi.y - qs.y, ez = pi.z - qs.z;
         return ex * ex + ey * ey + ez * ez;
     };
-    // FP64: the two comparisons of a test are decided in FP32 (from rounded
-    // positions) unless r^2 lies within the rounding of a cutoff for some lane;
-    // coordinates up to 2 Lc rounded to 2^-24 of it move r^2 by 5e-7 Lc near the
-    // cutoffs.  Some 124 FP64 tests per particle otherwise bound the build: 250 thousand particle cell 0.84 -> 0.15 ms
-    const float slack = 1e-5f + 8e-6f * fmaxf(sd.Lcf[0], fmaxf(sd.Lcf[1], sd.Lcf[2]));
+    // FP64: the two comparisons of a test are decided in FP32 (from rounded positions) unless r^2 lies within the
+    // rounding of a cutoff for some lane.  Some 124 FP64 tests per particle otherwise bound the build: 250 thousand
+    // particle cell 0.84 -> 0.15 ms
+    const float slack = sizeof(R) == 8 ? rounding_slack(sd) : 0.f;
     // ballots of r^2 < cut.x, cut.y for candidate q of lane; et: its list entry (FP64)
     auto inside = [&](const T4 &pi, const float4 &pf, const float4 &q, const float2 &cut, const uint32_t *et, bool pad,
                       unsigned &ma, unsigned &mi) {

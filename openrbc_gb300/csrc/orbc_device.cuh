@@ -146,9 +146,17 @@ __host__ __device__ __forceinline__ unsigned cell_code(const SysDev &s, int x, i
     return (tile << 6) | tile_spread2(unsigned(x) & 3u) | (tile_spread2(unsigned(y) & 3u) << 1) |
            (tile_spread2(unsigned(z) & 3u) << 2);
 }
-/* ids per system (tiles x 64) */
-__host__ __device__ __forceinline__ unsigned ncell_ids(const SysDev &s) {
-    return unsigned(s.ntile[0]) * unsigned(s.ntile[1]) * unsigned(s.ntile[2]) * 64u;
+/* FP64 forms decide r^2 < cut^2 in FP32 where that is safe: bound on the
+ * relative error that rounding puts into r^2 near a cutoff.  Each component of
+ * a distance takes at most five roundings of numbers up to 1.5 Lc in size, in
+ * sum 5 Lc 2^-24, so r is off by up to 5.2e-7 Lc and r^2 by 1.1e-6 Lc / cut (and 4e-7
+ * for its own arithmetic).  The cutoffs are 1.1225 and more, so 4e-6 Lc + 1e-5
+ * holds with a factor of four.  The expansion in the error needs it small
+ * against the cutoff: cells beyond 10^4 (an open system with a stray particle)
+ * are left to FP64. */
+__device__ __forceinline__ float rounding_slack(const SysDev &sd) {
+    const float L = fmaxf(sd.Lcf[0], fmaxf(sd.Lcf[1], sd.Lcf[2]));
+    return L < 1e4f ? 1e-5f + 4e-6f * L : __int_as_float(0x7f800000);
 }
 
 struct SysState {

@@ -236,7 +236,7 @@ template<class R> struct ShiftTab {
 template<> struct ShiftTab<double> {
     double v[3][32];
     float f[3][32];  // rounded, for the shell test
-    float slack;     // relative error bound of the rounded test
+    float slack;     // bound on the relative error of the rounded r^2 (rounding_slack)
 };
 template<class R> __device__ __forceinline__ void init_shift(const SysDev &sd, ShiftTab<R> &sh) {
     const int lane = threadIdx.x & 31;
@@ -246,15 +246,14 @@ template<class R> __device__ __forceinline__ void init_shift(const SysDev &sd, S
         sh.v[2][lane] = R(-(lane / 9 - 1)) * lc_of<R>(sd, 2);
         if constexpr (sizeof(R) == 8)
             for (int d = 0; d < 3; ++d) sh.f[d][lane] = float(sh.v[d][lane]);
-        // coordinates up to Lc, rounded to 2^-24 of it, put 2.4e-7 Lc of relative error into r^2 near the cutoffs
         if constexpr (sizeof(R) == 8)
-            if (lane == 0) sh.slack = 1e-5f + 4e-6f * fmaxf(sd.Lcf[0], fmaxf(sd.Lcf[1], sd.Lcf[2]));
+            if (lane == 0) sh.slack = rounding_slack(sd);
     }
     __syncwarp();
 }
 /* Whether the pair of a shell row is inside r^2 < lim, for the FP64 form: in
- * FP32 where the rounding of the coordinates cannot change the answer, and
- * by the FP64 distance in the thin shell that remains. */
+ * FP32 where the rounding of the coordinates cannot change the answer
+ * (rounding_slack), and by the FP64 distance in the thin shell that remains. */
 __device__ __forceinline__ bool shell_inside(const ShiftTab<double> &sh, const double4a &pi, const double4a &pj, int c,
                                              double lim) {
     const float fx = float(pi.x) - float(pj.x) + sh.f[0][c], fy = float(pi.y) - float(pj.y) + sh.f[1][c],

@@ -124,3 +124,34 @@ def test_fp64_decisions_at_the_cutoffs(types):
     if 4 in types or 5 in types:
         assert step > 1e-4  # an interaction that is cut off where it has not died out
     assert np.abs(f - f_ref)[ok].max() <= 1e-6 * step
+
+
+@pytest.mark.parametrize("stray", [1e8, 2e13])
+def test_fp64_in_cells_that_single_precision_cannot_resolve(stray):
+    """A particle far away makes the cells of its axis large: coordinates in
+    them, rounded to single precision, no longer tell which pairs are near."""
+    from openrbc_gb300 import RTParameter, Simulation
+    g = np.random.default_rng(5)
+    n = 400
+    k = np.arange(n)
+    x = np.stack([1.3 * (k % 20), 1.3 * (k // 20), np.zeros(n)], 1) + g.uniform(-0.1, 0.1, (n, 3))
+    far = np.concatenate([x, [[stray, 0.0, 0.0]]])
+    nrm = np.tile([0.0, 0.0, 1.0], (n + 1, 1))
+    nrm[:, 1] += 0.1 * np.sin(np.arange(n + 1))
+    nrm /= np.linalg.norm(nrm, axis=1)[:, None]
+    res = []
+    for p in (far, x):
+        m = len(p)
+        z = np.zeros((m, 3))
+        with Simulation(RTParameter(init="lipid", precision="fp64"), box=((-1e14, 1e14),) * 3, skin=0.4) as s:
+            s.upload(p, nrm[:m], z, z, np.zeros(m, np.int32), np.arange(1, m + 1, dtype=np.int32))
+            counts, lst = s.neighbors()
+            f, t, _ = s.forces()
+            res.append((counts[:n], f[:n], t[:n]))
+    # offsets in a cell of 1.5e10 resolve 1e-6; the list cutoff's neighbourhood is left out
+    d2 = ((x[:, None, :] - x[None, :, :]) ** 2).sum(2)
+    edge = (np.abs(np.sqrt(d2) - 3.0) < 1e-4).any(1)
+    assert np.array_equal(res[0][0][~edge], res[1][0][~edge])
+    scale = np.abs(res[1][1]).max()
+    assert np.abs(res[0][1] - res[1][1]).max() < 1e-4 * scale
+    assert np.abs(res[0][2] - res[1][2]).max() < 1e-4 * np.abs(res[1][2]).max()
