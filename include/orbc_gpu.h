@@ -333,19 +333,20 @@ typedef struct {
 } orbc_profile;
 int orbc_gpu_profile(orbc_handle *h, int nsteps, orbc_profile *out);
 
-/* Autotuner: times trial_steps graph-captured steps per candidate from a
- * snapshot of the current state, keeps the fastest, and restores the snapshot
- * (state, step counter, thermostat), so the simulation does not advance.
- * Dimensions, in order: the list-build form (bits 3-4) at the caller's skin;
- * neighbour-list skin (0.3, 0.45, 0.6, 0.8, 1.0) x force-loop form
- * (kernel_variant bits 0-1, and bit 5); the two skins half-way to the best
- * one's neighbours; the occupancy form (bit 2); the other list-build forms
- * again; and the rebuild cadence (rebuild_every 0 = only when a particle moved
- * more than skin/2, else also every 5 or 10 steps).  The forms run the same
- * kernels (see kernel_variant), so skin and cadence are what it decides.  Compensated accumulation (bit 6) is an accuracy
- * choice and is kept as the caller set it.  trials (may be NULL) receives up
- * to max_trials rows.  No reference counterpart (the reference's cadences are
- * fixed command-line values, src/runtime_parameter.h:57-60). */
+/* Autotuner: picks the neighbour-list skin and the rebuild cadence.  Each
+ * candidate is timed once, over 3 x trial_steps graph-captured steps from a
+ * snapshot of the current state; the fastest is kept and the snapshot (state,
+ * step counter, thermostat) restored, so the simulation does not advance.
+ * kernel_variant stays as the caller set it.  Rows, in order: the three
+ * list-build forms (kernel_variant bits 3-4) at the caller's skin; skin (0.3,
+ * 0.45, 0.6, 0.8, 1.0) x force-loop form (bits 0-1, and bit 5); the two skins
+ * half-way to the best one's neighbours; the occupancy form (bit 2); two
+ * list-build forms; and the rebuild cadence (rebuild_every 0 = only when a
+ * particle moved more than skin/2, else also every 5 or 10 steps).  The forms
+ * run the same kernels (see kernel_variant), so rows that differ in form alone
+ * repeat one measurement.  trials (may be NULL) receives up to max_trials
+ * rows.  No reference counterpart (the reference's cadences are fixed
+ * command-line values, src/runtime_parameter.h:57-60). */
 typedef struct {
     double skin;
     int variant;        /* kernel_variant of the trial */

@@ -1609,7 +1609,7 @@ template<class R> class Engine : public EngineBase {
         return ORBC_OK;
     }
 
-    /* Pick the neighbour-list skin and the force-kernel form by timing short
+    /* Pick the neighbour-list skin and the rebuild cadence by timing short
      * trials from one snapshot of the state; the snapshot (positions,
      * orientations, velocities, angular velocities, step counter, thermostat)
      * is restored afterwards, so tuning does not advance the simulation. */
@@ -1627,11 +1627,20 @@ template<class R> class Engine : public EngineBase {
         for (size_t k = 0; k < hss.size(); ++k) topo.descs[k].zeta = hss[k].zeta;
         const double skins[] = {0.3, 0.45, 0.6, 0.8, 1.0};
         double best_ms = 1e300, best_skin = P.skin;
-        int best_var = P.kernel_variant, best_every = P.rebuild_every, nt = 0;
-        const int keep = P.kernel_variant & 64;  // compensated accumulation: the caller's accuracy choice
-        auto trial = [&](double sk, int var, int every) -> int {
+        int best_every = P.rebuild_every, nt = 0;
+        // every (skin, cadence) is timed once, over the same number of steps
+        struct Timed {
+            double skin, ms, rebuilds;
+            int every;
+        };
+        std::vector<Timed> timed;
+        auto time_pair = [&](double sk, int every, Timed &t) -> int {
+            for (const Timed &q : timed)
+                if (q.skin == sk && q.every == every) {
+                    t = q;
+                    return ORBC_OK;
+                }
             P.skin = sk;
-            P.kernel_variant = var | keep;
             P.rebuild_every = every;
             int r = relayout(x, nv, v, o, hs.step);
             if (r) return r;
@@ -1639,57 +1648,64 @@ template<class R> class Engine : public EngineBase {
             if (r) return r;
             Scalars b4;
             CK(cudaMemcpy(&b4, Sd.p, sizeof(Scalars), cudaMemcpyDeviceToHost));
-            r = step(trial_steps, nullptr);
-            if (r) return r;
+            double ms = 0;
+            for (int k = 0; k < 3; ++k) {
+                r = step(trial_steps, nullptr);
+                if (r) return r;
+                ms += last_ms;
+            }
             Scalars af;
             CK(cudaMemcpy(&af, Sd.p, sizeof(Scalars), cudaMemcpyDeviceToHost));
-            const double ms = last_ms / trial_steps;
+            t = Timed{sk, ms / (3.0 * trial_steps), double(af.rebuilds - b4.rebuilds) / (3.0 * trial_steps), every};
+            timed.push_back(t);
+            return ORBC_OK;
+        };
+        const int keep = P.kernel_variant & 64;  // compensated accumulation: the caller's accuracy choice
+        auto trial = [&](double sk, int var, int every) -> int {
+            Timed t;
+            const int r = time_pair(sk, every, t);
+            if (r) return r;
             if (trials && nt < max_trials) {
                 trials[nt].skin = sk;
                 trials[nt].variant = var | keep;
                 trials[nt].rebuild_every = every;
-                trials[nt].ms_per_step = ms;
-                trials[nt].rebuilds_per_step = double(af.rebuilds - b4.rebuilds) / trial_steps;
+                trials[nt].ms_per_step = t.ms;
+                trials[nt].rebuilds_per_step = t.rebuilds;
             }
             ++nt;
-            if (ms < best_ms) {
-                best_ms = ms;
+            if (t.ms < best_ms) {
+                best_ms = t.ms;
                 best_skin = sk;
-                best_var = var | keep;
                 best_every = every;
             }
             return ORBC_OK;
         };
-        // skin and cadence are what the trials decide; the form bits that they
-        // also vary (list build 3-4, force loop 0-1 and 5, occupancy 2) select the
-        // same kernels, and the table of trials keeps its rows for callers that
-        // read it
-        const int occ0 = P.kernel_variant & 4, every0 = P.rebuild_every;
+        // The rows that vary a form bit alone (list build 3-4, force loop 0-1 and
+        // 5, occupancy 2) repeat their (skin, cadence): the forms select the same
+        // kernels, and the table keeps these rows for callers that read it
+        const int base = 3 | (P.kernel_variant & 4), every0 = P.rebuild_every;
         const double skin0 = P.skin;
         for (int f = 0; f < 3; ++f)
-            if ((rc = trial(skin0, 3 | occ0 | (f << 3), every0))) return rc;
-        const int rest = (best_var & 24) | occ0;
+            if ((rc = trial(skin0, base | (f << 3), every0))) return rc;
         const int loops[] = {0, 1, 2, 3, 3 | 32};
         for (double sk : skins)
             for (int lf : loops)
-                if ((rc = trial(sk, lf | rest, every0))) return rc;
-        const int nsk = int(sizeof(skins) / sizeof(skins[0]));
-        int bi = 0;
-        while (bi + 1 < nsk && skins[bi] != best_skin) ++bi;
-        const double lo_sk = 0.5 * (skins[bi > 0 ? bi - 1 : 0] + best_skin);
-        const double hi_sk = 0.5 * (skins[bi + 1 < nsk ? bi + 1 : nsk - 1] + best_skin);
-        const int bv = best_var & ~64;
-        if ((rc = trial(lo_sk, bv, every0))) return rc;
-        if ((rc = trial(hi_sk, bv, every0))) return rc;
-        if ((rc = trial(best_skin, (best_var & ~64) ^ 4, every0))) return rc;
-        const int lf = (best_var >> 3) & 3;
-        for (int f = 0; f < 3; ++f)
-            if (f != lf && (rc = trial(best_skin, (best_var & (7 | 32)) | (f << 3), every0))) return rc;
+                if ((rc = trial(sk, lf | (base & 4), every0))) return rc;
+        double below = best_skin, above = best_skin;  // the best skin's neighbours in the grid (itself at its ends)
+        for (double sk : skins) {
+            if (sk < best_skin) below = sk;
+            if (sk > best_skin && above == best_skin) above = sk;
+        }
+        const double lo_sk = 0.5 * (below + best_skin), hi_sk = 0.5 * (above + best_skin);
+        if ((rc = trial(lo_sk, base, every0))) return rc;
+        if ((rc = trial(hi_sk, base, every0))) return rc;
+        if ((rc = trial(best_skin, base ^ 4, every0))) return rc;
+        for (int f = 1; f < 3; ++f)
+            if ((rc = trial(best_skin, base | (f << 3), every0))) return rc;
         for (int every : {5, 10})
-            if (every != every0 && (rc = trial(best_skin, best_var & ~64, every))) return rc;
+            if (every != every0 && (rc = trial(best_skin, base, every))) return rc;
         if (ntrials) *ntrials = nt;
         P.skin = best_skin;
-        P.kernel_variant = best_var;
         P.rebuild_every = best_every;
         return relayout(x, nv, v, o, hs.step);
     }

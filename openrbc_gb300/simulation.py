@@ -264,9 +264,8 @@ class Simulation:
         return pr.as_dict()
 
     def autotune(self, trial_steps: int = 30):
-        """Pick skin, force-kernel and list-build forms and rebuild cadence by
-        timing trials (orbc_gpu_autotune); the state is restored afterwards.
-        Returns the trial table."""
+        """Pick skin and rebuild cadence by timing trials (orbc_gpu_autotune);
+        the state is restored afterwards.  Returns the trial table."""
         rows = (N.TuneTrial * 64)()
         nt = C.c_int()
         self._check(N.lib().orbc_gpu_autotune(self.h, int(trial_steps), rows, 64, C.byref(nt)))
