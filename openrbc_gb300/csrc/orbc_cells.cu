@@ -43,8 +43,7 @@ __device__ __forceinline__ int gate_closed(const int *gate) { return gate && !__
 /* stable in-tile ranking (warp match + per-warp digit counts) and scatter.  */
 /* ------------------------------------------------------------------------- */
 __global__ void __launch_bounds__(256) k_rs_hist(const uint32_t *keys, int64_t n, int shift, int *counts,
-                                                  int ntiles, const int *gate) {
-    if (gate_closed(gate)) return;
+                                                  int ntiles) {
     __shared__ int h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -58,8 +57,7 @@ __global__ void __launch_bounds__(256) k_rs_hist(const uint32_t *keys, int64_t n
     counts[int64_t(threadIdx.x) * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-__global__ void __launch_bounds__(1024) k_rs_scan(int *counts, int ntiles, int *digit_total, const int *gate) {
-    if (gate_closed(gate)) return;
+__global__ void __launch_bounds__(1024) k_rs_scan(int *counts, int ntiles, int *digit_total) {
     __shared__ int wsum[32];
     __shared__ int carry;
     int *row = counts + int64_t(blockIdx.x) * ntiles;
@@ -99,8 +97,7 @@ __global__ void __launch_bounds__(1024) k_rs_scan(int *counts, int ntiles, int *
 
 __global__ void __launch_bounds__(256) k_rs_scatter(const uint32_t *kin, const int *vin, uint32_t *kout, int *vout,
                                                      int64_t n, int shift, const int *counts, int ntiles,
-                                                     const int *digit_total, int *inv, const int *gate) {
-    if (gate_closed(gate)) return;
+                                                     const int *digit_total) {
     __shared__ int base_s[256];
     __shared__ int run[256];
     __shared__ int wcnt[8][256];
@@ -152,7 +149,6 @@ __global__ void __launch_bounds__(256) k_rs_scatter(const uint32_t *kin, const i
             const int pos = base_s[dg] + wcnt[warp][dg] + rank;
             kout[pos] = key;
             vout[pos] = val;
-            if (inv) inv[val] = pos;
         }
         __syncthreads();
     }
@@ -160,15 +156,15 @@ __global__ void __launch_bounds__(256) k_rs_scatter(const uint32_t *kin, const i
 
 int sort_tiles(int64_t n) { return int((n + SORT_TILE - 1) / SORT_TILE); }
 
-int radix_sort_pairs(uint32_t *keys[2], int *vals[2], int *counts, int *digit_total, int *inv, int64_t n,
-                     int passes, int ntiles, const int *gate, cudaStream_t st) {
+int radix_sort_pairs(uint32_t *keys[2], int *vals[2], int *counts, int *digit_total, int64_t n, int passes, int ntiles,
+                     cudaStream_t st) {
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
         const int shift = 8 * p;
-        k_rs_hist<<<ntiles, 256, 0, st>>>(keys[cur], n, shift, counts, ntiles, gate);
-        k_rs_scan<<<256, 1024, 0, st>>>(counts, ntiles, digit_total, gate);
+        k_rs_hist<<<ntiles, 256, 0, st>>>(keys[cur], n, shift, counts, ntiles);
+        k_rs_scan<<<256, 1024, 0, st>>>(counts, ntiles, digit_total);
         k_rs_scatter<<<ntiles, 256, 0, st>>>(keys[cur], vals[cur], keys[1 - cur], vals[1 - cur], n, shift, counts,
-                                             ntiles, digit_total, p == passes - 1 ? inv : nullptr, gate);
+                                             ntiles, digit_total);
         cur = 1 - cur;
     }
     return cur;

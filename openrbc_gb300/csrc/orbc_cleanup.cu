@@ -283,7 +283,7 @@ int launch_cleanup_mark(const KArgs<R> &a, int mingen, double tol2, double4a *ge
             k_cl_update<R><<<cl_blocks(int64_t(a.npad) * 32), 256, 0, st>>>(a, gen, mingen, a.skey[fin], a.sval[fin]);
         k_cl_assign<R><<<cl_blocks(a.npad), 256, 0, st>>>(a, gen, a.skey[0], a.sval[0], dr2);
         fin = radix_sort_pairs(const_cast<uint32_t **>(a.skey), const_cast<int **>(a.sval), a.counts, a.digit_total,
-                               nullptr, a.npad, 4, a.ntiles, nullptr, st);
+                               a.npad, 4, a.ntiles, st);
     }
     k_cl_mark<R><<<cl_blocks((int64_t(a.npad) + 1) * 32), 256, 0, st>>>(a, gen, mingen, a.skey[fin], a.sval[fin],
                                                                         dr2, tol2, gone_home, removed);

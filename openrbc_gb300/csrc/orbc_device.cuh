@@ -298,8 +298,8 @@ template<class R> void launch_download(const KArgs<R> &a, int64_t h0, int64_t h1
 void launch_set_cond(cudaGraphConditionalHandle h, Scalars *S, cudaStream_t st);
 void launch_morton(const double *p3, int64_t n, const double *bsize3, uint32_t *keys, cudaStream_t st);
 // LSD radix sort of (key, index) pairs, stable; returns the buffer index (0/1) holding the result.
-int radix_sort_pairs(uint32_t *keys[2], int *vals[2], int *counts, int *digit_total, int *inv, int64_t n,
-                     int passes, int ntiles, const int *gate, cudaStream_t st);
+int radix_sort_pairs(uint32_t *keys[2], int *vals[2], int *counts, int *digit_total, int64_t n, int passes, int ntiles,
+                     cudaStream_t st);
 int sort_tiles(int64_t n);
 constexpr int SORT_TILE = 4096;
 // message of the handle-less entry points, read back by orbc_gpu_error(NULL)

@@ -2205,7 +2205,7 @@ int orbc_gpu_morton_order(const double *p3, int64_t n, const double *bsize3, int
     if (e == cudaSuccess) {
         launch_morton(dp, n, bsize3, k[0], 0);
         k_iota<<<1216, 256>>>(v[0], n);
-        fin = radix_sort_pairs(k, v, cnt, tot, nullptr, n, 4, ntiles, nullptr, 0);
+        fin = radix_sort_pairs(k, v, cnt, tot, n, 4, ntiles, 0);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpy(order, v[fin], size_t(n) * sizeof(int), cudaMemcpyDeviceToHost);

@@ -136,7 +136,7 @@ extern "C" int orbc_gpu_morton_order_noalloc(const double *d_p3, int64_t n, cons
     // encoder, and every pass rewrites all digit counts and totals it reads
     launch_morton(d_p3, n, bsize3, keys[0], st);
     k_na_iota<<<int(std::min<int64_t>((n + 255) / 256, 1024)), 256, 0, st>>>(vals[0], n);
-    const int fin = radix_sort_pairs(keys, vals, counts, total, nullptr, n, 4, sort_tiles(n), nullptr, st);
+    const int fin = radix_sort_pairs(keys, vals, counts, total, n, 4, sort_tiles(n), st);
     // the launches' own errors (nothing was pending at entry)
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return na_fail("morton_order_noalloc: launch", e);

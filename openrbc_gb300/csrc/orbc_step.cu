@@ -75,10 +75,7 @@ __device__ __forceinline__ void inv_sqrt(float r2, float &r, float &rinv) {
  * y <- y (3 - r2 y^2) / 2, started from the FP32 hardware estimate.  The
  * relative error e goes to about 1.5 e^2 per step (1e-7 -> 2e-14 -> below
  * the FP64 rounding), so two steps leave only a few ulp of rounding; the
- * callers pass pair distances 1e-5 < r2 < 100, well inside the FP32 range.
- * It takes fewer FP64 operations than a correctly rounded square root and
- * division, which bound the plain FP64 step (3 % of its time on the 4.03M
- * cell; forces change by 9e-16 relative). */
+ * protein pairs that call it have 1e-5 < r2 < 7, well inside the FP32 range. */
 __device__ __forceinline__ void inv_sqrt(double r2, double &r, double &rinv) {
     double y = double(rsqrtf(float(r2)));
     y = y * (1.5 - 0.5 * r2 * y * y);
@@ -88,36 +85,6 @@ __device__ __forceinline__ void inv_sqrt(double r2, double &r, double &rinv) {
 }
 __device__ __forceinline__ float rnorm3(float x, float y, float z) { return rsqrtf(x * x + y * y + z * z); }
 __device__ __forceinline__ double rnorm3(double x, double y, double z) { return 1.0 / sqrt(x * x + y * y + z * z); }
-
-/* Anisotropic poly 4-8 pair seen from particle i (src/pairwise_kernel.h:30-68,
- * src/pairwise_kernel_fused.h:22-61).  dx = x_i - x_j. */
-template<class R, bool E>
-__device__ __forceinline__ void aniso(const PairP<R> &P, R dx, R dy, R dz, R r2, R nix, R niy, R niz, R njx, R njy,
-                                      R njz, R3<R> &f, R3<R> &t, R &e) {
-    R r, rinv;
-    inv_sqrt(r2, r, rinv);
-    const R ux = dx * rinv, uy = dy * rinv, uz = dz * rinv;
-    const R ninj = nix * njx + niy * njy + niz * njz;
-    const R niu = nix * ux + niy * uy + niz * uz;
-    const R nju = njx * ux + njy * uy + njz * uz;
-    const R A = R(1) + P.alpha * (ninj - niu * nju - R(1));
-    const R rc = P.cut - r;
-    const R rc3 = rc * rc * rc;
-    const R rc4 = rc * rc3;
-    const R rc7 = rc3 * rc4;
-    const R pix = nix - niu * ux, piy = niy - niu * uy, piz = niz - niu * uz;
-    const R pjx = njx - nju * ux, pjy = njy - nju * uy, pjz = njz - nju * uz;
-    const R alphaua = P.aatt * rc4;
-    const R alphauar = alphaua * rinv;
-    const R fra = P.rep8 * rc7 + A * P.att4 * rc3;
-    f.x += fra * ux + alphauar * (nju * pix + niu * pjx);
-    f.y += fra * uy + alphauar * (nju * piy + niu * pjy);
-    f.z += fra * uz + alphauar * (nju * piz + niu * pjz);
-    t.x -= alphaua * pjx;
-    t.y -= alphaua * pjy;
-    t.z -= alphaua * pjz;
-    if (E) e += R(0.5) * (P.rep * rc4 * rc4 + A * P.att * rc4);
-}
 
 /* Lennard-Jones with the WCA cut (src/pairwise_kernel_fused.h:63-77). */
 template<class R, bool E>
@@ -146,19 +113,15 @@ __device__ __forceinline__ void repf(const PairP<R> &P, R dx, R dy, R dz, R r2, 
     if (E) e += R(0.5) * P.rep * rc4 * rc4;
 }
 
-/* Dispatch of src/compute_pairwise_fused.h:91-236 for a non lipid-lipid pair. */
+/* Dispatch of src/compute_pairwise_fused.h:91-236 for a pair without an
+ * anisotropic interaction. */
 template<class R, bool E>
-__device__ __forceinline__ void pair_general(const PairP<R> &P, R dx, R dy, R dz, R r2, R nix, R niy, R niz,
-                                                  R njx, R njy, R njz, R3<R> &f, R3<R> &t, R &e) {
+__device__ __forceinline__ void pair_general(const PairP<R> &P, R dx, R dy, R dz, R r2, R3<R> &f, R &e) {
     if (!(r2 > R(1e-5))) return;
-    if (r2 < P.cutsq) {
-        if (P.kind == PAIR_ANISO)
-            aniso<R, E>(P, dx, dy, dz, r2, nix, niy, niz, njx, njy, njz, f, t, e);
-        else
-            repf<R, E>(P, dx, dy, dz, r2, f, e);
-    } else if (r2 < P.ljcutsq) {
+    if (r2 < P.cutsq)
+        repf<R, E>(P, dx, dy, dz, r2, f, e);
+    else if (r2 < P.ljcutsq)
         ljf<R, E>(P, dx, dy, dz, r2, f, e);
-    }
 }
 __device__ __forceinline__ int wrap_delta(int d, int n) {
     if (2 * d >= n) return d - n;
@@ -542,15 +505,14 @@ __device__ __forceinline__ void pair_sums(const KArgs<R> &a, const FFDev<R> &F, 
             const int k = __ffs(int(hb)) - 1;
             hb &= hb - 1u;
             const uint32_t ent = __ldg(shell - int64_t(k + k0) * 32);
-            const T4 pj = ldg4<R>(pos + (ent & NB_MASK)), nj = ldg4<R>(nrm + (ent & NB_MASK));
+            const T4 pj = ldg4<R>(pos + (ent & NB_MASK));
             R d[3], ee = 0;
             offset(ent, pj, d);
-            R3<R> df = {0, 0, 0}, dt = {0, 0, 0};
-            pair_general<R, E>(F.pair[ty * NT + w_type(wbits(pj.w))], d[0], d[1], d[2], dist2(d), ni.x, ni.y, ni.z,
-                               nj.x, nj.y, nj.z, df, dt, ee);
-            const R v[6] = {df.x, df.y, df.z, dt.x, dt.y, dt.z};
+            R3<R> df = {0, 0, 0};
+            pair_general<R, E>(F.pair[ty * NT + w_type(wbits(pj.w))], d[0], d[1], d[2], dist2(d), df, ee);
+            const R v[3] = {df.x, df.y, df.z};
 #pragma unroll
-            for (int q = 0; q < 6; ++q) {
+            for (int q = 0; q < 3; ++q) {
                 if (K)
                     kahan_add(A.s[q], A.c[K ? q : 0], v[q]);
                 else
