@@ -572,9 +572,8 @@ def main():
     fp64 = None
     ferr = None
     if not args.skip_fp64 and args.fp64_steps > 0:
-        # the mixed run's force-loop and list-build forms and skin; the
-        # occupancy form (bit 2) is sized for FP32 registers and compensated
-        # accumulation (bit 6) is an FP32 remedy: both are left out
+        # the mixed run's skin; compensated accumulation (bit 6) is an FP32
+        # remedy and is left out (the other form bits select nothing)
         form = (tune["chosen"]["variant"] if tune else args.form) & ~(4 | 64)
         skin = tune["chosen"]["skin"] if tune else (args.skin if args.skin is not None else SKIN)
         sim64 = make_sim(w, "fp64", skin=skin, kernel_variant=form)

@@ -484,7 +484,7 @@ template<class R> __device__ __forceinline__ void nlist_finalise(const KArgs<R> 
  * SW warps share 32 slots, each taking 32 / SW of their particles: one warp's
  * chain of cells, ballots and expansions is some 80 thousand cycles long, which
  * is the time of the build while the GPU is not full. */
-// Bound by instruction issue (61 % of peak) and each warp's chain.  1.0M-particle
+// Bound by instruction issue (69 % of peak) and each warp's chain; FP64: by the FP64 pipe (86 %).  1.0M-particle
 // cell 0.357 -> 0.266 ms, 4.03M 1.34 -> 0.98, 1.0M lipids in 23 vesicles 0.359 ->
 // 0.279 against table lookups, searched staging and blocks of four warps; a third
 // copy of phase 1 for lipids alone made the cell with anchors slower (0.379 ms:

@@ -267,7 +267,7 @@ template<class R> __global__ void k_cleanup_apply(KArgs<R> a, const int *newidx,
     if (blockIdx.x == 0 && threadIdx.x == 0) a.S->rebuild = 1;
 }
 
-int cl_blocks(int64_t threads) { return int(std::min<int64_t>((threads + 255) / 256, 152 * 16)); }
+int cl_blocks(int64_t threads) { return int(std::min<int64_t>((threads + 255) / 256, NUM_SM * 16)); }
 
 }  // namespace
 

@@ -61,7 +61,7 @@ template<class R> __global__ void k_set_carried(KArgs<R> a, const double *f3, co
 
 int io_grid(int64_t n) {
     const int64_t g = (n + 255) / 256;
-    return int(g < 1 ? 1 : (g > 152 * 8 ? 152 * 8 : g));
+    return int(g < 1 ? 1 : (g > NUM_SM * 8 ? NUM_SM * 8 : g));
 }
 
 }  // namespace

@@ -1428,9 +1428,9 @@ template<class R> void reduce_sums(const KArgs<R> &a, int mode, int count_step, 
  * to 97 thousand slots), where the chain of dependent gathers sets the time
  * and nothing else competes for the registers; beyond that two, whose 16
  * resident blocks hide more than the longer batch does.  Step kernel, batches
- * of two / four: 2,048 particles 18.8 / 15.4 us, 32,768: 20.9 / 18.3 us, 131,946:
- * 29 / 34 us, 1.0M: 174 / 243 us.  FP64: one row (the FP64 pipe is the bound:
- * 1.11 against 1.13 and 1.15 ms on a 250 thousand particle cell). */
+ * of two / four: 2,048 particles 19.1 / 17.8 us, 32,768: 20.1 / 18.5 us, 97,000: 21.9 /
+ * 22.2 us, 131,946: 31.4 / 36.5 us, 1.0M: 166 / 199 us.  FP64: one row (the FP64 pipe is
+ * the bound: 0.84 against 0.88 and 0.92 ms on a 250 thousand particle cell). */
 template<class R, class L> void by_batch(const KArgs<R> &a, L launch) {
     const int nb = a.npad / force_threads<R>;
     if constexpr (sizeof(R) == 8)
