@@ -261,7 +261,7 @@ extern "C" int orbc_gpu_place_lipids(const double *vert3, int64_t nvert, const i
     a.x = dx;
     a.n = dn;
     a.failed = dfail;
-    const int64_t warps = std::min<int64_t>(nface, int64_t(NUM_SM) * 64);
+    const int64_t warps = std::min<int64_t>(nface, int64_t(orbc::NUM_SM) * 64);
     k_place_lipids<<<unsigned((warps + 3) / 4), 128>>>(a);
     int failed = 0;
     cudaError_t e = cudaMemcpy(&failed, dfail, sizeof(int), cudaMemcpyDeviceToHost);
