@@ -263,6 +263,11 @@ __device__ __forceinline__ bool apart(double r2) {
     const long long b = __double_as_longlong(r2);
     return b > __double_as_longlong(1e-5) && b <= 0x7ff0000000000000LL;
 }
+/* infinite or not a number, and +-0, on the integer pipe for the same reason */
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_int(x) & 0x7f800000) == 0x7f800000; }
+__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+__device__ __forceinline__ bool is_zero(float x) { return (__float_as_int(x) << 1) == 0; }
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
 __device__ __forceinline__ float positive_part(float x) { return fmaxf(x, 0.f); }
 __device__ __forceinline__ double positive_part(double x) { return __double2hiint(x) < 0 ? 0.0 : x; }
 
@@ -641,9 +646,8 @@ __device__ __forceinline__ void slot_forces(const KArgs<R> &a, const FFDev<R> &F
     if (!(P.cut > R(0))) na.x = na.y = na.z = R(0);
     const T4 *__restrict__ pos = a.pos[cur], *__restrict__ nrm = a.nrm[cur];
     pair_sums<R, E, K, U, false>(a, F, P, i, pos, nrm, ty, packed, pi, na, sh, A);
-    const R sum = add_rn(add_rn(add_rn(A.s[0], A.s[1]), add_rn(A.s[2], A.s[3])),
-                         add_rn(add_rn(A.s[4], A.s[5]), A.s[6]));
-    if (__any_sync(0xffffffffu, sum != sum)) {
+    // (a normal that is not a number or infinite makes the coefficient of d and so every component of f one)
+    if (__any_sync(0xffffffffu, not_finite(A.s[0]))) {
         // again with the pairs in range alone.  What the sums take is read anew: kept in registers until here,
         // it would cost the common path spills
         asm volatile("" ::: "memory");
@@ -651,7 +655,7 @@ __device__ __forceinline__ void slot_forces(const KArgs<R> &a, const FFDev<R> &F
         A.clear();
         pair_sums<R, E, K, 1, true>(a, F, own_params(pl2), i, pos, nrm, ty, __ldcg(a.nnb + i), pi, na, sh, A);
     }
-    if (A.s[6] == R(0)) na.x = na.y = na.z = R(0);
+    if (is_zero(A.s[6])) na.x = na.y = na.z = R(0);
     if (K) {
 #pragma unroll
         for (int k = 0; k < NACC; ++k) A.s[k] = add_rn(A.s[k], -A.c[K ? k : 0]);
